@@ -273,7 +273,9 @@ TBTKKPM_API int tbtkkpm_matrix_set_config(
  * bulk-copy kernel with a ring of S stages per warp and W warps per block;
  * 10000 + 1000*S + 10*WMAX + W a cp.async-staged kernel.  Real-vector
  * kernels (real matrices at the mixed precisions): cap + 100*8 (802, 803)
- * keeps the doubling dot sums in shared memory instead of registers.
+ * keeps the doubling dot sums in shared memory instead of registers;
+ * 100000 + 1000000*CV + 1000*R + 10*CW + BPS a tile-staged step of R-row
+ * tiles (CV 200: FP64 on vectors of doubles, for a real matrix's sums).
  * (No reference counterpart.) */
 TBTKKPM_API int tbtkkpm_step_configs(int precision, int ldos, int *out, int cap);
 
@@ -282,7 +284,10 @@ TBTKKPM_API int tbtkkpm_step_configs(int precision, int ldos, int *out, int cap)
  * run on real float vectors instead of complex64 ones: every Chebyshev
  * vector of a real matrix started from basis vectors is real, and the real
  * kernels give the same moments (value, 0) with half the vector bytes.
- * The FP64 precision keeps complex128 vectors (the reference's data).
+ * The FP64 precision takes vectors of doubles where the call returns sums
+ * over the moments (ldos, density), with the same values; moments handed to
+ * the caller come from complex128 vectors, the reference's data, whose zeros
+ * carry signs.  FP64 results that overflow are those of complex128 vectors.
  * set_real(m, 0) turns the real vectors off (1, the default, allows them);
  * tbtkkpm_matrix_real reports whether the values are real and whether the
  * real vectors are in use; tbtkkpm_matrix_step_configs lists the step

@@ -85,6 +85,7 @@ struct TilePlan {
   uint32_t umax, wmax;     // most distinct outside columns / entries per row of a tile
   uint32_t nruns;          // runs of all tiles
   uint32_t pairs;          // row-pair plan: entries of [w][R/2] row pairs, two values each
+  uint32_t unit;           // columns staged together (2: for vector rows of 8 bytes)
 };
 
 // Byte layout of one shared-memory ring stage of a tile-staged step
@@ -142,8 +143,8 @@ struct tbtkkpm_matrix {
   // autotuned step configuration per (kernel class, padded batch width):
   // {threads per row, values per thread, min blocks per SM}
   std::map<uint64_t, std::array<int, 3>> tuned;
-  // tile plans by (rows per tile, complex values, row pairs): key
-  // 1024*pairs + 2*R + complex
+  // tile plans by (rows per tile, complex values, row pairs, staging unit):
+  // key 2048*(unit - 1) + 1024*pairs + 2*R + complex
   std::map<int, tbtkkpm::TilePlanStore> plans;
   std::mutex lock;
   void release_all() {
@@ -201,6 +202,11 @@ int energy_sum_host(tbtkkpm_table *t, const double *mu, uint32_t K, int type, vo
 int ldos_sites_terms(tbtkkpm_matrix *m, tbtkkpm_table *t, uint32_t M, const uint32_t *sites,
                      uint32_t B, double broadening, int precision, double *ldos_out,
                      double *err_out);
+// tbtkkpm_moments_batched; real64_ok: the caller does not see the signs of
+// zero moments, so FP64 moments of a real matrix may come from real vectors.
+int moments_pairs(tbtkkpm_matrix *m, const uint32_t *from, uint32_t B, const uint32_t *to,
+                  const uint32_t *to_owner, uint32_t K, uint32_t M, double broadening, int precision,
+                  bool real64_ok, double *mu_out, double *err_out);
 // Lorentz damping numerators a[n] and denominator b (host libm).
 void damping_factors(uint32_t M, double broadening, std::vector<double> &a, double &b);
 // Error estimate of doubled moments against the directly gathered ones.
@@ -216,8 +222,10 @@ double ldos_error_estimate(double moment_err, double wmax, const double *row, ui
 void doubling_error(const std::vector<double2> &mu, const std::vector<double2> &direct,
                     uint32_t K, uint32_t M, uint32_t ld, double *err);
 // The matrix's gather plan for R-row tiles (real or complex values; pairs:
-// the row-pair plan of complex values, R >= 16), built on first use; *out is
-// null when some tile is too large for the builder.
-int tile_plan(tbtkkpm_matrix *m, int R, bool cplx, const TilePlan **out, bool pairs = false);
+// the row-pair plan of complex values, R >= 16; unit 2: columns staged in
+// pairs, real values and R = 64), built on first use; *out is null when some
+// tile is too large for the builder.
+int tile_plan(tbtkkpm_matrix *m, int R, bool cplx, const TilePlan **out, bool pairs = false,
+              uint32_t unit = 1);
 
 }  // namespace tbtkkpm

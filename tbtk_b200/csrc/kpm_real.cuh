@@ -295,10 +295,11 @@ kpm_step_real(Sell A, uint32_t Bp, const float *__restrict__ x, float *__restric
 
 // Sets x[from_b][b] = 1 for each source (x zeroed beforehand) and the zeroth
 // moments, as kpm_init_sources.
-static __global__ void kpm_init_sources_real(uint32_t B, uint32_t Bp, const uint32_t *from,
-                                             float *x, Targets tg) {
+template <typename T>
+__global__ void kpm_init_sources_real(uint32_t B, uint32_t Bp, const uint32_t *from, T *x,
+                                      Targets tg) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < B) x[(uint64_t)from[i] * Bp + i] = 1.0f;
+  if (i < B) x[(uint64_t)from[i] * Bp + i] = T(1);
   if (i < tg.count) {
     const uint32_t b = tg.col[i];
     const double v = (tg.row[i] == from[b]) ? 1.0 : 0.0;

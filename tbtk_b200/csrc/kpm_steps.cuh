@@ -22,7 +22,8 @@ enum StepClass : int {
   kClassMixed = 1,
   kClassMixedDots = 2,
   kClassMixedReal = 3,
-  kClassMixedRealDots = 4
+  kClassMixedRealDots = 4,
+  kClassFP64Real = 5  // FP64 on vectors of doubles (a real matrix); listed with kClassFP64
 };
 
 struct StepArgs {
@@ -181,11 +182,13 @@ void launch_async(cudaStream_t st, int device, unsigned max_grid, const StepArgs
 
 // Tile-staged step variants: 100000 + 1000000*CV + 1000*R + 10*CW + BPS
 // (CV the widening split of kpm_step_tiled, plus 100 for the row-pair
-// form, R rows per tile, CW consumer warps, BPS blocks per SM).
+// form, 200 for the FP64 steps on real vectors, R rows per tile, CW consumer
+// warps, BPS blocks per SM).
 constexpr int kTiledVariant = 100000;
+constexpr int kTiledReal64 = 200;
 inline bool is_tiled_variant(int v) { return v >= kTiledVariant; }
 inline int tiled_rows(int v) { return ((v - kTiledVariant) % 1000000) / 1000; }
-inline bool tiled_pairs(int v) { return (v - kTiledVariant) / 1000000 >= 100; }
+inline bool tiled_pairs(int v) { return (v - kTiledVariant) / 1000000 / 100 == 1; }
 inline int tiled_bps(int v) { return v % 10; }
 
 template <bool CPLX, int TPR, int VPT, int R, int CW, int BPS, bool FIRST, bool DOTS, int CV,
@@ -196,7 +199,11 @@ void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs
   using Val = typename TiledTypes<CPLX, F64>::Val;
   auto kern = kpm_step_tiled<CPLX, TPR, VPT, R, CW, BPS, FIRST, DOTS, CV, F64>;
   *grid = 0;
-  if (!a.plan || a.plan->R != (uint32_t)R || a.plan->pairs != (CV >= 100 ? 1u : 0u)) return;
+  // columns staged together: two for rows of 8 bytes (the copies' 16-byte rule)
+  constexpr uint32_t unit = TPR * VPT * sizeof(E) < 16 ? 2u : 1u;
+  if (!a.plan || a.plan->R != (uint32_t)R || a.plan->pairs != (CV >= 100 ? 1u : 0u) ||
+      a.plan->unit != unit)
+    return;
   const TilePlan &p = *a.plan;
   const TiledLayout ly =
       tiled_layout(p, a.Bp * (uint32_t)sizeof(E), (uint32_t)sizeof(Val), tiled_budget(BPS));
@@ -228,6 +235,12 @@ void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs
   {CLS, T, P, kTiledVariant + 1000 * R + 10 * CW + BPS,                              \
    &launch_tiled<true, T, P, R, CW, BPS, true, false, 0, true>,                      \
    &launch_tiled<true, T, P, R, CW, BPS, false, false, 0, true>}
+
+// the same on vectors of doubles, for a real matrix
+#define TBTKKPM_TILED_ENTRY_F64_REAL(T, P, R, CW, BPS)                               \
+  {kClassFP64Real, T, P, kTiledVariant + 1000000 * kTiledReal64 + 1000 * R + 10 * CW + BPS, \
+   &launch_tiled<false, T, P, R, CW, BPS, true, false, 0, true>,                     \
+   &launch_tiled<false, T, P, R, CW, BPS, false, false, 0, true>}
 
 extern const StepEntry kStepsFP64[];
 extern const int kNumStepsFP64;

@@ -101,7 +101,7 @@ __device__ __forceinline__ double f2d_scaled(float x) {
 constexpr double kWideUp = 0x1p896;
 
 // Element type of a vector row and value type of an entry (F64: the
-// complex128 vectors of the FP64 recursion).
+// vectors of the FP64 recursion, complex128, or double for a real matrix).
 template <bool CPLX, bool F64 = false> struct TiledTypes;
 template <> struct TiledTypes<false, false> {
   using E = float;
@@ -114,6 +114,47 @@ template <> struct TiledTypes<true, false> {
 template <> struct TiledTypes<true, true> {
   using E = double2;
   using Val = double2;
+};
+template <> struct TiledTypes<false, true> {
+  using E = double;
+  using Val = double;
+};
+
+// The VPT doubles a thread owns in a row of a real FP64 batch, as RPack:
+// chunks of 16 bytes (one double for VPT = 1), interleaved over the group.
+template <int TPR, int VPT> struct DPack {
+  static constexpr int CS = VPT < 2 ? 1 : 2;
+  static constexpr int NL = VPT / CS;
+  static_assert(VPT % CS == 0, "real FP64 packs are 8 B or multiples of 16 B");
+  using L = typename std::conditional<CS == 1, double, double2>::type;
+  __device__ __forceinline__ static uint32_t col_of(int sub, int j) {
+    return (uint32_t)(((j / CS) * TPR + sub) * CS + j % CS);
+  }
+  __device__ __forceinline__ static int slot_of(int sub, uint32_t c) {
+    const uint32_t p = c / CS;
+    return (int)(p % TPR) == sub ? (int)(p / TPR) * CS + (int)(c % CS) : -1;
+  }
+  __device__ __forceinline__ static void load_rw(const double *row, int sub, L (&o)[NL]) {
+    const L *q = reinterpret_cast<const L *>(row);
+#pragma unroll
+    for (int j = 0; j < NL; j++) o[j] = q[j * TPR + sub];
+  }
+  __device__ __forceinline__ static double get(const L (&o)[NL], int j) {
+    if constexpr (CS == 1) {
+      return o[j];
+    } else {
+      const double2 f = o[j >> 1];
+      return (j & 1) ? f.y : f.x;
+    }
+  }
+  __device__ __forceinline__ static void store(double *row, int sub, const double (&v)[VPT]) {
+    L *q = reinterpret_cast<L *>(row);
+#pragma unroll
+    for (int j = 0; j < NL; j++) {
+      if constexpr (CS == 1) q[j * TPR + sub] = v[j];
+      else q[j * TPR + sub] = make_double2(v[2 * j], v[2 * j + 1]);
+    }
+  }
 };
 
 // One recursion step over the tiles of `P` (same outputs as kpm_step_real
@@ -132,11 +173,19 @@ template <> struct TiledTypes<true, true> {
 // row still sees its own entries in CSR order.  Every choice gives the same
 // stored vectors.
 //
-// F64 (complex, CV 0, no dot products): the FP64 recursion on complex128
-// vectors in the reference's operation order (Exact64: each row's sum starts
-// at -j_{n-1} and adds every complex product, each rounded once, in CSR
-// order, Lib/src/Solver/ChebyshevExpander.cpp:171-186), the same as
+// F64 (CV 0, no dot products): the FP64 recursion in the reference's
+// operation order (Exact64: each row's sum starts at -j_{n-1} and adds every
+// complex product, each rounded once, in CSR order,
+// Lib/src/Solver/ChebyshevExpander.cpp:171-186), the same as
 // kpm_step<double2, Exact64>: moments bit-identical to the reference's.
+// CPLX runs it on complex128 vectors.  Without CPLX (a real matrix, unit
+// vectors as sources) every imaginary part of the complex recursion is a
+// zero and a product's real part v.re*x.re - 0*0 is v.re*x.re, so the real
+// parts alone, on vectors of doubles, give the same moments (a zero's sign
+// aside) from 10 bytes an entry instead of 18 and half the vector bytes.
+// That holds while every value is finite; a recursion that overflows (a
+// scale factor below the spectrum) leaves a moment that is not, and the
+// caller repeats it on complex vectors.
 template <bool CPLX, int TPR, int VPT, int R, int CW, int BPS, bool FIRST, bool DOTS, int CV = 0,
           bool F64 = false>
 __global__ void __launch_bounds__(32 * (CW + 1), BPS)
@@ -148,7 +197,7 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
   using Val = typename TiledTypes<CPLX, F64>::Val;
   using Pk = typename std::conditional<
       CPLX, typename std::conditional<F64, Pack<double2, TPR, VPT>, Pack<float2, TPR, VPT>>::type,
-      RPack<TPR, VPT>>::type;
+      typename std::conditional<F64, DPack<TPR, VPT>, RPack<TPR, VPT>>::type>::type;
   using L = typename Pk::L;
   constexpr int NL = Pk::NL;
   constexpr bool PAIR = CV >= 100;
@@ -159,7 +208,7 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
   constexpr int PASSES = ((int)EW + RPP - 1) / RPP;
   static_assert(CW * 32 % TPR == 0, "a row group must divide the consumer threads");
   static_assert(!PAIR || (CPLX && R >= 16), "row pairs: complex vectors, 16-byte slot chunks");
-  static_assert(!F64 || (CPLX && CV == 0 && !DOTS), "FP64 steps: complex values, every moment direct");
+  static_assert(!F64 || (CV == 0 && !DOTS), "FP64 steps: every moment direct");
   extern __shared__ __align__(128) unsigned char tsm[];
   uint64_t *full = reinterpret_cast<uint64_t *>(tsm);
   uint64_t *empty = full + kTiledMaxStages;
@@ -210,8 +259,10 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
       const uint32_t r0 = t * R, Rt = min((uint32_t)R, P.N - r0);
       // pair entries carry two values each: w * R values either way
       const uint32_t ebytes = w * R * (uint32_t)sizeof(Val), sbytes = w * EW * 2u;
-      const uint32_t bytes =
-          ebytes + sbytes + (Rt + nuniq + (FIRST ? 0u : Rt)) * rowbytes;
+      // rows of 8 bytes: the last tile's own rows may be odd, its copies take
+      // the buffer's padding row too (runs come in whole plan units)
+      const uint32_t obytes = rowbytes < 16u ? align_up(Rt * rowbytes, 16) : Rt * rowbytes;
+      const uint32_t bytes = ebytes + sbytes + nuniq * rowbytes + (FIRST ? 1u : 2u) * obytes;
       if (lane == 0) mbar_expect_tx(&full[s], bytes);
       __syncwarp();
       const uint64_t e0 = (uint64_t)h0.x * EW;
@@ -220,9 +271,9 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
           bulk_load(st, static_cast<const Val *>(P.eval) + e0 * (PAIR ? 2 : 1), ebytes, &full[s]);
         if (lane == 1) bulk_load(st + LY.off_slots, P.eslot + e0, sbytes, &full[s]);
       }
-      if (lane == 2) bulk_load(st + LY.off_xs, x + (uint64_t)r0 * Bp, Rt * rowbytes, &full[s]);
+      if (lane == 2) bulk_load(st + LY.off_xs, x + (uint64_t)r0 * Bp, obytes, &full[s]);
       if (!FIRST && lane == 3)
-        bulk_load(st + LY.off_prev, y + (uint64_t)r0 * Bp, Rt * rowbytes, &full[s]);
+        bulk_load(st + LY.off_prev, y + (uint64_t)r0 * Bp, obytes, &full[s]);
       for (uint32_t c = 0; c < nruns; c += 32) {
         uint2 rn = run0;
         if (c > 0) rn = (c + lane < nruns) ? __ldg(P.runs + h0.y + c + lane) : make_uint2(0, 0);
@@ -271,7 +322,45 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
       const E *prev = reinterpret_cast<const E *>(st + LY.off_prev);
 #pragma unroll
       for (int p = 0; p < PASSES; p++) {
-        if constexpr (F64) {
+        if constexpr (F64 && !CPLX) {
+          const uint32_t lr = grp + p * RPP;
+          if (lr >= Rt) continue;
+          const uint32_t row = r0 + lr;
+          double acc[VPT];
+          if constexpr (FIRST) {
+#pragma unroll
+            for (int j = 0; j < VPT; j++) acc[j] = 0.0;
+          } else {
+            L yv[NL];
+            Pk::load_rw(reinterpret_cast<const double *>(prev) + (size_t)lr * Bp, sub, yv);
+#pragma unroll
+            for (int j = 0; j < VPT; j++) acc[j] = -Pk::get(yv, j);
+          }
+          for (uint32_t k = 0; k < w; k++) {
+            const uint16_t sl = slots[k * R + lr];
+            if (sl == kSlotPad) break;
+            double v = vals[k * R + lr];
+            if constexpr (FIRST) v = v * 0.5;
+            L xr[NL];
+            Pk::load_rw(reinterpret_cast<const double *>(xs) + (size_t)sl * Bp, sub, xr);
+#pragma unroll
+            for (int j = 0; j < VPT; j++) acc[j] = __dadd_rn(acc[j], __dmul_rn(v, Pk::get(xr, j)));
+          }
+          if ((bw[p] >> (row & 31)) & 1u) {
+            for (uint32_t q = target_first(tg, row); q < tg.count && __ldg(tg.row + q) == row; q++) {
+              const int jt = Pk::slot_of(sub, __ldg(tg.col + q));
+              if (jt >= 0) {
+#pragma unroll
+                for (int j = 0; j < VPT; j++)
+                  if (j == jt)
+                    tg.mu[(uint64_t)__ldg(tg.out + q) * tg.ld + n_out] = make_double2(acc[j], 0.0);
+              }
+            }
+          }
+          Pk::store(reinterpret_cast<double *>(y) + (uint64_t)row * Bp, sub, acc);
+          continue;
+        }
+        if constexpr (F64 && CPLX) {
           const uint32_t lr = grp + p * RPP;
           if (lr >= Rt) continue;
           const uint32_t row = r0 + lr;
@@ -466,7 +555,7 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
               d_np[j] += PA ? f2d_scaled(np) : (double)np;
             }
           }
-        } else if constexpr (!CPLX) {
+        } else if constexpr (!CPLX && !F64) {
           double acc[VPT];
           if constexpr (FIRST) {
 #pragma unroll
@@ -565,8 +654,14 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
 // the runs of consecutive ones counted (k_plan_count) or listed
 // (k_plan_fill).  A tile with more than kPlanCap entries sets *bad.
 
-// Loads the tile's outside columns into keys[0, n2) (n2 = next power of two
-// of the entry count, padded with kPad) and sorts them ascending.
+// UNIT is the number of columns staged together: 1, or 2 for vector rows of
+// 8 bytes, whose copies would otherwise break the 16-byte rule.  A unit is
+// the columns [UNIT*i, UNIT*(i + 1)); runs and slots are in columns.
+
+// Loads the units of the tile's outside columns (each by its first column)
+// into keys[0, n2) (n2 = next power of two of the entry count, padded with
+// kPad) and sorts them ascending.
+template <uint32_t UNIT>
 __device__ inline uint32_t plan_sort_tile(uint32_t *keys, const uint32_t *col, uint32_t e0,
                                           uint32_t T, uint32_t r0, uint32_t r1) {
   uint32_t n2 = 1;
@@ -575,7 +670,7 @@ __device__ inline uint32_t plan_sort_tile(uint32_t *keys, const uint32_t *col, u
     uint32_t k = kPad;
     if (i < T) {
       const uint32_t c = col[e0 + i];
-      k = (c >= r0 && c < r1) ? kPad : c;
+      k = (c >= r0 && c < r1) ? kPad : c - c % UNIT;
     }
     keys[i] = k;
   }
@@ -598,13 +693,14 @@ __device__ inline uint32_t plan_sort_tile(uint32_t *keys, const uint32_t *col, u
   return n2;
 }
 
-// flags of sorted position i: bit 0 a new distinct column, bit 1 the start
-// of a run of consecutive columns
+// flags of sorted position i: bit 0 a new distinct unit, bit 1 the start
+// of a run of consecutive units
+template <uint32_t UNIT>
 __device__ __forceinline__ uint32_t plan_flags(const uint32_t *keys, uint32_t i) {
   const uint32_t k = keys[i];
   if (k == kPad) return 0;
   if (i > 0 && keys[i - 1] == k) return 0;
-  const bool run = i == 0 || keys[i - 1] != k - 1;
+  const bool run = i == 0 || keys[i - 1] != k - UNIT;
   return 1u | (run ? 2u : 0u);
 }
 
@@ -631,7 +727,7 @@ __device__ inline uint32_t plan_block_scan(uint32_t v, uint32_t *total) {
   return before + inc - v;
 }
 
-template <int R>
+template <int R, uint32_t UNIT = 1>
 __global__ void __launch_bounds__(kPlanBlock)
 k_plan_count(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
              const uint32_t *__restrict__ col, uint32_t *tw, uint32_t *truns, uint32_t *tuniq,
@@ -649,10 +745,10 @@ k_plan_count(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
       continue;
     }
     if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
-    const uint32_t n2 = plan_sort_tile(pkeys, col, e0, T, r0, r1);
+    const uint32_t n2 = plan_sort_tile<UNIT>(pkeys, col, e0, T, r0, r1);
     uint32_t nu = 0, nr = 0, wmax = 0;
     for (uint32_t i = threadIdx.x; i < n2; i += blockDim.x) {
-      const uint32_t f = plan_flags(pkeys, i);
+      const uint32_t f = plan_flags<UNIT>(pkeys, i);
       nu += f & 1u;
       nr += f >> 1;
     }
@@ -663,10 +759,10 @@ k_plan_count(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
     atomicMax(&cnt[2], wmax);
     __syncthreads();
     if (threadIdx.x == 0) {
-      tuniq[t] = cnt[0];
+      tuniq[t] = cnt[0] * UNIT;
       truns[t] = cnt[1];
       tw[t] = cnt[2];
-      atomicMax(&maxes[0], cnt[0]);
+      atomicMax(&maxes[0], cnt[0] * UNIT);
       atomicMax(&maxes[1], cnt[2]);
     }
     __syncthreads();
@@ -707,7 +803,7 @@ k_plan_pair_width(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowp
   }
 }
 
-template <int R, bool CPLX, bool PAIRS = false>
+template <int R, bool CPLX, bool PAIRS = false, uint32_t UNIT = 1>
 __global__ void __launch_bounds__(kPlanBlock)
 k_plan_fill(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
             const uint32_t *__restrict__ col, const double2 *__restrict__ val,
@@ -724,14 +820,14 @@ k_plan_fill(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
     const uint32_t r0 = t * R, r1 = min(r0 + R, N);
     const uint32_t e0 = rowptr[r0], T = rowptr[r1] - e0;
     if (T > kPlanCap) continue;  // the count kernel flagged it; the plan is not used
-    const uint32_t w = tw[t], nruns = truns[t], nuniq = tuniq[t];
+    const uint32_t w = tw[t], nruns = truns[t], nuniq = tuniq[t], units = nuniq / UNIT;
     if (threadIdx.x == 0) hdr[t] = make_uint4(ent_begin[t], run_begin[t], nuniq, w | (nruns << 16));
-    const uint32_t n2 = plan_sort_tile(pkeys, col, e0, T, r0, r1);
-    // distinct columns and run starts in sorted order
+    const uint32_t n2 = plan_sort_tile<UNIT>(pkeys, col, e0, T, r0, r1);
+    // distinct units and run starts in sorted order
     uint32_t ubase = 0, rbase = 0;
     for (uint32_t b = 0; b < n2; b += blockDim.x) {
       const uint32_t i = b + threadIdx.x;
-      const uint32_t f = i < n2 ? plan_flags(pkeys, i) : 0u;
+      const uint32_t f = i < n2 ? plan_flags<UNIT>(pkeys, i) : 0u;
       uint32_t ut, rt;
       const uint32_t up = plan_block_scan(f & 1u, &ut);
       const uint32_t rp = plan_block_scan(f >> 1, &rt);
@@ -743,18 +839,19 @@ k_plan_fill(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
     __syncthreads();
     for (uint32_t q = threadIdx.x; q < nruns; q += blockDim.x) {
       const uint32_t u = rstart[q];
-      const uint32_t len = (q + 1 < nruns ? rstart[q + 1] : nuniq) - u;
-      runs[run_begin[t] + q] = make_uint2(uniq[u], (u << 16) | len);
+      const uint32_t len = (q + 1 < nruns ? rstart[q + 1] : units) - u;
+      runs[run_begin[t] + q] = make_uint2(uniq[u], (u * UNIT) << 16 | len * UNIT);
     }
     // the shared-memory slot of column c (own rows first, then the runs)
     auto slot_of = [&](uint32_t c) -> uint32_t {
       if (c >= r0 && c < r1) return c - r0;
-      uint32_t lo = 0, hi = nuniq;
+      const uint32_t first = c - c % UNIT;
+      uint32_t lo = 0, hi = units;
       while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (uniq[mid] < c) lo = mid + 1; else hi = mid;
+        if (uniq[mid] < first) lo = mid + 1; else hi = mid;
       }
-      return R + lo;
+      return R + lo * UNIT + c % UNIT;
     };
     if constexpr (PAIRS) {
       // entries: [w][R/2] of {slot | rows << 14} and two values (zero for

@@ -21,15 +21,15 @@ namespace {
 using cplx = std::complex<double>;
 
 // G_NonPrincipal[k][e] of the pairs (to[k], from[owner[k]]) over the table's
-// energies.
+// energies.  real64_ok: see moments_pairs.
 int greens_np(tbtkkpm_matrix *m, tbtkkpm_table *t, const std::vector<uint32_t> &from,
               const std::vector<uint32_t> &to, const std::vector<uint32_t> &owner,
-              double broadening, int precision, std::vector<cplx> &G) {
+              double broadening, int precision, std::vector<cplx> &G, bool real64_ok = false) {
   const uint32_t K = (uint32_t)to.size(), M = t->M;
   std::vector<cplx> mu((size_t)K * M);
-  int rc = tbtkkpm_moments_batched(m, from.data(), (uint32_t)from.size(), to.data(), owner.data(),
-                                   K, M, broadening, precision,
-                                   reinterpret_cast<double *>(mu.data()), nullptr);
+  int rc = tbtkkpm::moments_pairs(m, from.data(), (uint32_t)from.size(), to.data(), owner.data(), K,
+                                  M, broadening, precision, real64_ok,
+                                  reinterpret_cast<double *>(mu.data()), nullptr);
   if (rc) return rc;
   G.assign((size_t)K * t->E, cplx(0, 0));
   return tbtkkpm_greens(t, reinterpret_cast<const double *>(mu.data()), K, TBTKKPM_NONPRINCIPAL,
@@ -91,7 +91,8 @@ extern "C" int tbtkkpm_density(tbtkkpm_matrix *m, tbtkkpm_table *t, const uint32
   std::vector<uint32_t> from(sites, sites + S), to(sites, sites + S), owner(S);
   for (uint32_t s = 0; s < S; s++) owner[s] = s;
   std::vector<cplx> G;
-  if ((rc = greens_np(m, t, from, to, owner, broadening, precision, G))) return rc;
+  // only imag(G) of diagonal pairs enters, never a zero: real vectors serve
+  if ((rc = greens_np(m, t, from, to, owner, broadening, precision, G, true))) return rc;
   const uint32_t E = t->E;
   for (uint32_t s = 0; s < S; s++) {
     // data[offset] += weight*imag(G[e])/M_PI*dE

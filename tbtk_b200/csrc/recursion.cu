@@ -40,6 +40,17 @@ bool real_mode(const tbtkkpm_matrix *m, int precision) {
   return is_mixed(precision) && m->values_real && m->use_real;
 }
 
+// FP64 batches of a real matrix may run on vectors of doubles
+// (kpm_step_tiled with F64 and without CPLX) under the same setting.  Their
+// moments equal the complex recursion's except for the signs of zeros, which
+// the complex sums carry along (a conjugated real amplitude has an imaginary
+// part of -0), so they serve the calls that return sums over the moments
+// (LDOS, density), where a zero's sign drops out; moments handed to the
+// caller come from complex vectors.
+bool real64_mode(const tbtkkpm_matrix *m, int precision) {
+  return !is_mixed(precision) && m->values_real && m->use_real;
+}
+
 // The register-staged shape of a batch (kpm_step / kpm_step_real): the
 // fallback of the tile-staged defaults below, and the default of widths the
 // tile-staged steps do not serve.
@@ -98,6 +109,29 @@ Shape register_shape_for(int precision, uint32_t B, bool real, bool dots) {
 // Tile-staged variant: 100000 + 1000000*CV + 1000*R + 10*CW + BPS.
 constexpr int tiled(int cv, int rows, int cw, int bps) {
   return 100000 + 1000000 * cv + 1000 * rows + 10 * cw + bps;
+}
+
+// FP64 steps on real vectors (kClassFP64Real).
+constexpr int tiled64r(int rows, int cw, int bps) { return tiled(kTiledReal64, rows, cw, bps); }
+
+// Default FP64 shape of a real matrix, {0, 0} where the complex steps stay.
+// us per step on the 2048^2 lattice (best of the complex steps in brackets)
+// for B = 1 / 2 / 4 / 8: 94 (170) / 122 (223) / 184 (345) / 317 (667), for
+// B = 16 / 32 / 64 / 128: 532 (1385) / 967 (2138) / 2047 (4207) / 4081
+// (8386); at 131k rows 8.2 (9.1) / 10 (14) / 13 (27) / 18 (41) / 41 (73) / 73
+// (141) for B = 4 ... 128, at 16k rows 6.2 (8.2) / 8.2 (10.3) / 10.3 (14.2)
+// for B = 16 / 32 / 64 and even below.  A single source is faster on the
+// complex thread per row up to 65k rows (5.1 against 6.2 us) and even at
+// 131k.
+Shape real64_shape_for(uint32_t B, uint32_t N) {
+  if (B <= 1) return N <= (1u << 17) ? Shape{0, 0} : Shape{1, 1, tiled64r(256, 8, 3)};
+  if (B <= 2) return {1, 2, tiled64r(256, 8, 3)};
+  if (B <= 4) return {1, 4, tiled64r(64, 2, 8)};
+  if (B <= 8) return {4, 2, tiled64r(64, 8, 4)};
+  if (B <= 16) return {8, 2, tiled64r(64, 8, 3)};
+  if (B <= 32) return {8, 4, tiled64r(32, 8, 3)};
+  if (B <= 64) return {8, 8, tiled64r(16, 8, 2)};
+  return {16, 8, tiled64r(8, 8, 2)};
 }
 
 // Default shape of a batch.  At mixed precision from 32 sources on (from 16
@@ -218,19 +252,21 @@ ShapeKey shape_key(const tbtkkpm_matrix *m, int cls, uint32_t Bp) {
 // for this (class, padded width), this process's choice for a matrix of the
 // same shape, or the default shape with MINB 2.
 const StepEntry *pick_step(const tbtkkpm_matrix *m, int precision, bool dots, uint32_t B,
-                           const StepEntry *force) {
+                           const StepEntry *force, bool real64) {
   if (force) return force;
   const bool real = real_mode(m, precision);
   const int cls = step_class(precision, dots, real);
-  const Shape s = shape_for(precision, B, real, dots, m->N);
-  auto it = m->tuned.find(tune_key(cls, s.bp()));
+  Shape s = shape_for(precision, B, real, dots, m->N);
+  if (real64 && real64_shape_for(B, m->N).bp()) s = real64_shape_for(B, m->N);
+  const int key = real64 ? kClassFP64Real : cls;
+  auto it = m->tuned.find(tune_key(key, s.bp()));
   if (it != m->tuned.end()) {
     const StepEntry *e = find_step(cls, it->second[0], it->second[1], it->second[2]);
     if (e) return e;
   }
   {
     std::lock_guard<std::mutex> lk(g_tuned_mu);
-    auto git = g_tuned.find(shape_key(m, cls, s.bp()));
+    auto git = g_tuned.find(shape_key(m, key, s.bp()));
     if (git != g_tuned.end()) {
       const StepEntry *e = find_step(cls, git->second[0], git->second[1], git->second[2]);
       if (e) return e;
@@ -240,30 +276,40 @@ const StepEntry *pick_step(const tbtkkpm_matrix *m, int precision, bool dots, ui
 }
 
 // A tile-staged entry runs with the matrix's plan for its tile height when
-// a ring of at least two stages fits its shared memory.  Otherwise a forced
+// a ring of at least two stages fits its shared memory; one on real FP64
+// vectors also needs the batch to take them (real64).  Otherwise a forced
 // entry is refused (TBTKKPM_ERR_UNSUPPORTED, which the autotuner skips) and
-// a chosen one gives way to the register-staged default of the batch.
-int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool forced,
+// a chosen one gives way: real FP64 vectors to the complex default, a
+// tile-staged step to the register-staged default of the batch.
+int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool forced, bool real64,
                   const StepEntry *&fn, const TilePlan *&plan) {
   plan = nullptr;
-  if (!fn || !is_tiled_variant(fn->minb)) return TBTKKPM_OK;
-  const bool cplx = !(fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots);
-  const TilePlan *p = nullptr;
-  int rc = tile_plan(m, tiled_rows(fn->minb), cplx, &p, tiled_pairs(fn->minb));
-  if (rc) return rc;
-  const uint32_t esz = fn->cls == kClassFP64 ? sizeof(double2) : cplx ? sizeof(float2) : sizeof(float);
-  const uint32_t vsz = cplx ? sizeof(double2) : sizeof(double);
-  if (p && tiled_layout(*p, (uint32_t)(fn->tpr * fn->vpt) * esz, vsz,
-                        tiled_budget(tiled_bps(fn->minb))).stages) {
-    plan = p;
-    return TBTKKPM_OK;
+  while (fn && is_tiled_variant(fn->minb)) {
+    const bool r64 = fn->cls == kClassFP64Real;
+    const bool cplx = !(r64 || fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots);
+    const uint32_t esz = fn->cls == kClassFP64 ? sizeof(double2)
+                         : r64                 ? sizeof(double)
+                         : cplx                ? sizeof(float2)
+                                               : sizeof(float);
+    const uint32_t vsz = cplx ? sizeof(double2) : sizeof(double);
+    const uint32_t rowbytes = (uint32_t)(fn->tpr * fn->vpt) * esz;
+    const TilePlan *p = nullptr;
+    if (!r64 || real64) {
+      int rc = tile_plan(m, tiled_rows(fn->minb), cplx, &p, tiled_pairs(fn->minb), rowbytes < 16 ? 2 : 1);
+      if (rc) return rc;
+    }
+    if (p && tiled_layout(*p, rowbytes, vsz, tiled_budget(tiled_bps(fn->minb))).stages) {
+      plan = p;
+      return TBTKKPM_OK;
+    }
+    if (forced)
+      return fail(TBTKKPM_ERR_UNSUPPORTED,
+                  "recursion: the tile-staged step %d x %d / %d does not fit this matrix", fn->tpr,
+                  fn->vpt, fn->minb);
+    const Shape s = r64 ? shape_for(precision, B, false, dots, m->N)
+                        : register_shape_for(precision, B, !cplx, dots);
+    fn = find_step(step_class(precision, dots, !cplx && !r64), s.tpr, s.vpt, s.minb);
   }
-  if (forced)
-    return fail(TBTKKPM_ERR_UNSUPPORTED,
-                "recursion: the tile-staged step %d x %d / %d does not fit this matrix", fn->tpr,
-                fn->vpt, fn->minb);
-  const Shape s = register_shape_for(precision, B, !cplx, dots);
-  fn = find_step(fn->cls, s.tpr, s.vpt, s.minb);
   return TBTKKPM_OK;
 }
 
@@ -279,23 +325,31 @@ struct TargetList {
 // identities, while the directly gathered moments of steps 0..M/2 land in
 // ws.mu_direct ([K][M/2+1]) for the error estimate.  A mixed doubling run
 // on a structurally symmetric matrix takes its first steps in FP64 on the
-// rows they reach (kpm_prefix) unless `head` is false.
+// rows they reach (kpm_prefix) unless `head` is false.  use_real64: an FP64
+// run of a real matrix takes real vectors; a moment that comes out infinite
+// or NaN then may differ from the complex recursion's, so the caller looks
+// at the moments (or at energy sums over them) and repeats such a run with
+// use_real64 false.
 int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &from,
               const TargetList &tl, uint32_t K, uint32_t M, bool doubling,
-              const StepEntry *force = nullptr, bool head = true) {
+              const StepEntry *force = nullptr, bool head = true, bool use_real64 = false) {
   Workspace &ws = m->ws;
   cudaStream_t st = m->stream;
   const uint32_t B = (uint32_t)from.size();
-  const StepEntry *fn = pick_step(m, precision, doubling, B, force);
+  const bool real64 = use_real64 && real64_mode(m, precision);
+  const StepEntry *fn = pick_step(m, precision, doubling, B, force, real64);
   const TilePlan *plan = nullptr;
-  int rc0 = resolve_tiled(m, precision, doubling, B, force != nullptr, fn, plan);
+  int rc0 = resolve_tiled(m, precision, doubling, B, force != nullptr, real64, fn, plan);
   if (rc0) return rc0;
   if (!fn) return fail(TBTKKPM_ERR_UNSUPPORTED, "no recursion kernel for batch %u", B);
   const uint32_t Bp = (uint32_t)(fn->tpr * fn->vpt);
   if (Bp < B) return fail(TBTKKPM_ERR_ARGUMENT, "configuration of %u columns for %u sources", Bp, B);
   const bool real = fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots;
-  const size_t esize = real ? sizeof(float) : (is_mixed(precision) ? sizeof(float2) : sizeof(double2));
-  const size_t vbytes = (size_t)m->N * Bp * esize;
+  const size_t esize = real ? sizeof(float)
+                       : is_mixed(precision) ? sizeof(float2)
+                       : fn->cls == kClassFP64Real ? sizeof(double) : sizeof(double2);
+  // rows of 8 bytes are staged two at a time: one padding row for an odd N
+  const size_t vbytes = (size_t)m->N * Bp * esize + (Bp * esize < 16 ? 16 : 0);
   const size_t words = ((size_t)m->N + 31) / 32;
   const uint32_t T = (uint32_t)tl.row.size();
   const uint32_t steps = doubling ? M / 2 : (M >= 2 ? M - 1 : 0);  // last j index computed
@@ -401,6 +455,9 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
     // the head wrote j_q, j_{q-1} and the moments through step q
   } else if (real) {
     kpm_init_sources_real<<<ib, 256, 0, st>>>(B, Bp, ws.from.as<uint32_t>(), ws.vec[0].as<float>(),
+                                              tg);
+  } else if (fn->cls == kClassFP64Real) {
+    kpm_init_sources_real<<<ib, 256, 0, st>>>(B, Bp, ws.from.as<uint32_t>(), ws.vec[0].as<double>(),
                                               tg);
   } else if (is_mixed(precision)) {
     kpm_init_sources<float2><<<ib, 256, 0, st>>>(B, Bp, ws.from.as<uint32_t>(),
@@ -554,12 +611,20 @@ uint32_t batch_width_for(const tbtkkpm_matrix *m, int precision, bool doubling) 
   return maxb;
 }
 
+// Whether no value of v is infinite or NaN (0 * v is NaN for those).
+static bool all_finite(const double *v, size_t n) {
+  double s = 0;
+  for (size_t i = 0; i < n; i++) s += 0.0 * v[i];
+  return s == 0;
+}
+
 // Moments of several batches: sources split into batches of at most
 // batch_width_for sources; to-indices follow their owner.  Results land in host
-// memory mu_out ([K][M]) undamped.
+// memory mu_out ([K][M]) undamped.  real64_ok: the signs of zero moments do
+// not matter to the caller (see real64_mode).
 static int moments_host(tbtkkpm_matrix *m, const uint32_t *from, uint32_t B, const uint32_t *to,
                         const uint32_t *owner, uint32_t K, uint32_t M, int precision,
-                        double *mu_out) {
+                        bool real64_ok, double *mu_out) {
   const uint32_t maxb = batch_width_for(m, precision, false);
   std::vector<std::vector<uint32_t>> by_owner(B);
   for (uint32_t k = 0; k < K; k++) by_owner[owner[k]].push_back(k);
@@ -586,17 +651,22 @@ static int moments_host(tbtkkpm_matrix *m, const uint32_t *from, uint32_t B, con
       tl.out.push_back(it[2]);
     }
     const uint32_t Kb = (uint32_t)global_k.size();
-    int rc = run_batch(m, precision, fr, tl, Kb, M, false);
-    if (rc) return rc;
     mu_host.resize((size_t)Kb * M);
-    m->timer.mark(m->stream, 2);
-    m->timer.mark(m->stream, 3);
-    cudaError_t e = cudaMemcpyAsync(mu_host.data(), m->ws.mu.ptr, sizeof(double2) * Kb * M,
-                                    cudaMemcpyDeviceToHost, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "moments: download");
-    m->timer.collect();
-    if ((rc = check_device_flag(m))) return rc;
+    for (bool real64 = real64_ok;; real64 = false) {
+      int rc = run_batch(m, precision, fr, tl, Kb, M, false, nullptr, true, real64);
+      if (rc) return rc;
+      m->timer.mark(m->stream, 2);
+      m->timer.mark(m->stream, 3);
+      cudaError_t e = cudaMemcpyAsync(mu_host.data(), m->ws.mu.ptr, sizeof(double2) * Kb * M,
+                                      cudaMemcpyDeviceToHost, m->stream);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
+      if (e != cudaSuccess) return cuda_fail(e, "moments: download");
+      m->timer.collect();
+      if ((rc = check_device_flag(m))) return rc;
+      if (!real64 || !real64_mode(m, precision) ||
+          all_finite(reinterpret_cast<const double *>(mu_host.data()), 2 * (size_t)Kb * M))
+        break;
+    }
     for (uint32_t i = 0; i < Kb; i++)
       std::memcpy(mu_out + 2 * (size_t)global_k[i] * M, mu_host.data() + (size_t)i * M,
                   sizeof(double2) * M);
@@ -653,7 +723,7 @@ extern "C" int tbtkkpm_moments(tbtkkpm_matrix *m, uint32_t from, const uint32_t 
   std::lock_guard<std::mutex> lk(m->lock);
   DeviceGuard g(m->device);
   std::vector<uint32_t> owner(K, 0u);
-  rc = moments_host(m, &from, 1, to, owner.data(), K, M, TBTKKPM_FP64, mu_out);
+  rc = moments_host(m, &from, 1, to, owner.data(), K, M, TBTKKPM_FP64, false, mu_out);
   if (rc) return rc;
   damp_host(K, M, broadening, mu_out);
   return TBTKKPM_OK;
@@ -663,6 +733,13 @@ extern "C" int tbtkkpm_moments_batched(tbtkkpm_matrix *m, const uint32_t *from, 
                                        const uint32_t *to, const uint32_t *to_owner, uint32_t K,
                                        uint32_t M, double broadening, int precision,
                                        double *mu_out, double *err_out) {
+  return tbtkkpm::moments_pairs(m, from, B, to, to_owner, K, M, broadening, precision, false, mu_out,
+                                err_out);
+}
+
+int tbtkkpm::moments_pairs(tbtkkpm_matrix *m, const uint32_t *from, uint32_t B, const uint32_t *to,
+                           const uint32_t *to_owner, uint32_t K, uint32_t M, double broadening,
+                           int precision, bool real64_ok, double *mu_out, double *err_out) {
   int rc = check_precision(precision);
   if (rc) return rc;
   if (K && !to_owner) return fail(TBTKKPM_ERR_ARGUMENT, "moments_batched: NULL to_owner");
@@ -671,7 +748,7 @@ extern "C" int tbtkkpm_moments_batched(tbtkkpm_matrix *m, const uint32_t *from, 
   if (K == 0) return TBTKKPM_OK;
   std::lock_guard<std::mutex> lk(m->lock);
   DeviceGuard g(m->device);
-  rc = moments_host(m, from, B, to, to_owner, K, M, precision, mu_out);
+  rc = moments_host(m, from, B, to, to_owner, K, M, precision, real64_ok, mu_out);
   if (rc) return rc;
   damp_host(K, M, broadening, mu_out);
   if (err_out)
@@ -1035,43 +1112,49 @@ int tbtkkpm::ldos_sites_terms(tbtkkpm_matrix *m, tbtkkpm_table *t, uint32_t M, c
       tl.col.push_back(it[1]);
       tl.out.push_back(it[1]);
     }
-    if ((rc = run_batch(m, precision, fr, tl, nb, M, doubling))) return rc;
     const uint32_t ld = M / 2 + 1;
-    if (doubling && err_out) {
-      // undamped moments for the estimate
-      mu_h.resize((size_t)nb * M);
-      direct_h.resize((size_t)nb * ld);
-      cudaMemcpyAsync(mu_h.data(), ws.mu.ptr, sizeof(double2) * nb * M, cudaMemcpyDeviceToHost,
-                      m->stream);
-      cudaMemcpyAsync(direct_h.data(), ws.mu_direct.ptr, sizeof(double2) * nb * ld,
-                      cudaMemcpyDeviceToHost, m->stream);
-    }
-    if (doubling) {
-      // Moments n <= M/2 were gathered directly as well; those carry less
-      // rounding than the dot-product identities, so they replace the
-      // doubled values, which remain only past M/2 where the damping
-      // sinh(lambda(1-n/M))/sinh(lambda) shrinks their weight.
-      e = cudaMemcpy2DAsync(ws.mu.ptr, sizeof(double2) * M, ws.mu_direct.ptr,
-                            sizeof(double2) * ld, sizeof(double2) * std::min(ld, M), nb,
-                            cudaMemcpyDeviceToDevice, m->stream);
-      if (e != cudaSuccess) return cuda_fail(e, "ldos_sites: direct moments");
-    }
-    m->timer.mark(m->stream, 2);
-    if (damp) {
-      kpm_damp<<<blocks_for((uint64_t)nb * M), 256, 0, m->stream>>>(nb, M, ws.damp.as<double>(), b,
-                                                                   ws.mu.as<double2>());
-      count_launches(1);
-    }
-    if ((rc = launch_energy_sum(m->stream, t, ws.mu.as<double2>(), nb, 4, ws.out.ptr, M))) return rc;
-    m->timer.mark(m->stream, 3);
-    e = cudaMemcpyAsync(ldos_out + (size_t)b0 * E, ws.out.ptr, sizeof(double) * (size_t)nb * E,
+    for (bool real64 = true;; real64 = false) {
+      if ((rc = run_batch(m, precision, fr, tl, nb, M, doubling, nullptr, true, real64))) return rc;
+      if (doubling && err_out) {
+        // undamped moments for the estimate
+        mu_h.resize((size_t)nb * M);
+        direct_h.resize((size_t)nb * ld);
+        cudaMemcpyAsync(mu_h.data(), ws.mu.ptr, sizeof(double2) * nb * M, cudaMemcpyDeviceToHost,
+                        m->stream);
+        cudaMemcpyAsync(direct_h.data(), ws.mu_direct.ptr, sizeof(double2) * nb * ld,
                         cudaMemcpyDeviceToHost, m->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "ldos_sites: download");
-    // one synchronisation per batch of up to 256 sites (seconds of work at
-    // full size): timers, the error estimate and the device status
-    if ((e = cudaStreamSynchronize(m->stream)) != cudaSuccess) return cuda_fail(e, "ldos_sites");
-    m->timer.collect();
-    if ((rc = check_device_flag(m))) return rc;
+      }
+      if (doubling) {
+        // Moments n <= M/2 were gathered directly as well; those carry less
+        // rounding than the dot-product identities, so they replace the
+        // doubled values, which remain only past M/2 where the damping
+        // sinh(lambda(1-n/M))/sinh(lambda) shrinks their weight.
+        e = cudaMemcpy2DAsync(ws.mu.ptr, sizeof(double2) * M, ws.mu_direct.ptr,
+                              sizeof(double2) * ld, sizeof(double2) * std::min(ld, M), nb,
+                              cudaMemcpyDeviceToDevice, m->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "ldos_sites: direct moments");
+      }
+      m->timer.mark(m->stream, 2);
+      if (damp) {
+        kpm_damp<<<blocks_for((uint64_t)nb * M), 256, 0, m->stream>>>(nb, M, ws.damp.as<double>(), b,
+                                                                     ws.mu.as<double2>());
+        count_launches(1);
+      }
+      if ((rc = launch_energy_sum(m->stream, t, ws.mu.as<double2>(), nb, 4, ws.out.ptr, M))) return rc;
+      m->timer.mark(m->stream, 3);
+      e = cudaMemcpyAsync(ldos_out + (size_t)b0 * E, ws.out.ptr, sizeof(double) * (size_t)nb * E,
+                          cudaMemcpyDeviceToHost, m->stream);
+      if (e != cudaSuccess) return cuda_fail(e, "ldos_sites: download");
+      // one synchronisation per batch of up to 256 sites (seconds of work at
+      // full size): timers, the error estimate and the device status
+      if ((e = cudaStreamSynchronize(m->stream)) != cudaSuccess) return cuda_fail(e, "ldos_sites");
+      m->timer.collect();
+      if ((rc = check_device_flag(m))) return rc;
+      // a sum over a moment that is not finite is not finite either
+      if (!real64 || !real64_mode(m, precision) ||
+          all_finite(ldos_out + (size_t)b0 * E, (size_t)nb * E))
+        break;
+    }
     if (err_out) {
       if (doubling) {
         doubling_error(mu_h, direct_h, nb, M, ld, err_out + b0);
@@ -1122,15 +1205,19 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   const StepEntry *t;
   int n;
   step_table(cls, &t, &n);
-  const StepEntry *best = nullptr;
-  double best_ms = 0;
+  // a real matrix's FP64 calls choose among the real and the complex steps
+  // where a sum is returned (real64_mode), among the complex ones elsewhere
+  const bool real64 = ldos && real64_mode(m, precision);
+  const StepEntry *best = nullptr, *best_cplx = nullptr;
+  double best_ms = 0, best_cplx_ms = 0;
   for (int i = 0; i < n; i++) {
     if ((uint32_t)(t[i].tpr * t[i].vpt) != Bp) continue;
+    if (t[i].cls == kClassFP64Real && !real64) continue;
     double ms = 0;
     bool skip = false;
     for (int rep = 0; rep < 2; rep++) {
       m->timer.recursion_ms = 0;
-      if ((rc = run_batch(m, precision, fr, tl, B, M, doubling, &t[i], false))) {
+      if ((rc = run_batch(m, precision, fr, tl, B, M, doubling, &t[i], false, real64))) {
         // a tile-staged step whose ring does not fit this matrix
         if (rc == TBTKKPM_ERR_UNSUPPORTED && is_tiled_variant(t[i].minb)) {
           rc = TBTKKPM_OK;
@@ -1154,6 +1241,10 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
       best = &t[i];
       best_ms = ms;
     }
+    if (t[i].cls != kClassFP64Real && (!best_cplx || ms < best_cplx_ms)) {
+      best_cplx = &t[i];
+      best_cplx_ms = ms;
+    }
   }
   const bool created = saved.ev[0] == nullptr;
   if (created) m->timer.destroy();
@@ -1166,11 +1257,14 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   }
   if (rc) return rc;
   if (!best) return fail(TBTKKPM_ERR_UNSUPPORTED, "matrix_autotune: no configuration for %u", B);
-  m->tuned[tune_key(cls, Bp)] = {best->tpr, best->vpt, best->minb};
-  {
+  auto keep = [&](int key, const StepEntry *e) {
+    if (!e) return;
+    m->tuned[tune_key(key, Bp)] = {e->tpr, e->vpt, e->minb};
     std::lock_guard<std::mutex> lk(g_tuned_mu);
-    g_tuned[shape_key(m, cls, Bp)] = {best->tpr, best->vpt, best->minb};
-  }
+    g_tuned[shape_key(m, key, Bp)] = {e->tpr, e->vpt, e->minb};
+  };
+  if (real64) keep(kClassFP64Real, best);
+  keep(cls, real64 ? best_cplx : best);
   if (tpr) *tpr = best->tpr;
   if (vpt) *vpt = best->vpt;
   if (minb) *minb = best->minb;
@@ -1194,6 +1288,7 @@ extern "C" int tbtkkpm_matrix_set_config(tbtkkpm_matrix *m, uint32_t B, int prec
                 "for %u columns", tpr, vpt, minb, Bp);
   std::lock_guard<std::mutex> lk(m->lock);
   m->tuned[tune_key(cls, Bp)] = {tpr, vpt, minb};
+  if (cls == kClassFP64) m->tuned[tune_key(kClassFP64Real, Bp)] = {tpr, vpt, minb};
   return TBTKKPM_OK;
 }
 

@@ -12,10 +12,10 @@ namespace tbtkkpm {
 
 namespace {
 
-template <int R>
+template <int R, uint32_t UNIT = 1>
 int count_tiles(cudaStream_t st, const tbtkkpm_matrix *m, uint32_t ntiles, unsigned grid,
                 DevBuf &tw, DevBuf &truns, DevBuf &tuniq, DevBuf &flags) {
-  k_plan_count<R><<<grid, kPlanBlock, kPlanCap * 4, st>>>(
+  k_plan_count<R, UNIT><<<grid, kPlanBlock, kPlanCap * 4, st>>>(
       m->N, ntiles, m->rowptr.as<uint32_t>(), m->col.as<uint32_t>(), tw.as<uint32_t>(),
       truns.as<uint32_t>(), tuniq.as<uint32_t>(), flags.as<unsigned>(), flags.as<unsigned>() + 2);
   return TBTKKPM_OK;
@@ -30,11 +30,11 @@ int pair_width(cudaStream_t st, const tbtkkpm_matrix *m, uint32_t ntiles, unsign
   return TBTKKPM_OK;
 }
 
-template <int R, bool CPLX, bool PAIRS = false>
+template <int R, bool CPLX, bool PAIRS = false, uint32_t UNIT = 1>
 int fill_tiles(cudaStream_t st, const tbtkkpm_matrix *m, uint32_t ntiles, unsigned grid,
                const DevBuf &ent, const DevBuf &run, const DevBuf &tw, const DevBuf &truns,
                const DevBuf &tuniq, TilePlanStore &p) {
-  auto kern = k_plan_fill<R, CPLX, PAIRS>;
+  auto kern = k_plan_fill<R, CPLX, PAIRS, UNIT>;
   constexpr int smem = 3 * kPlanCap * 4;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return cuda_fail(e, "tile plan: shared memory");
@@ -46,8 +46,12 @@ int fill_tiles(cudaStream_t st, const tbtkkpm_matrix *m, uint32_t ntiles, unsign
   return TBTKKPM_OK;
 }
 
-// pairs: the row-pair plan of complex values (R >= 16; k_plan_pair_width)
-int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, TilePlanStore &p) {
+// pairs: the row-pair plan of complex values (R >= 16; k_plan_pair_width);
+// unit: columns staged together (2: real values in tiles of 64 rows and up).
+// Tiles of 128 and 256 rows: real values only.
+int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, TilePlanStore &p) {
+  if (unit != 1 && (unit != 2 || cplx || pairs || R < 64))
+    return fail(TBTKKPM_ERR_UNSUPPORTED, "tile plan: no builder for units of %u columns", unit);
   if (pairs && (!cplx || R < 16))
     return fail(TBTKKPM_ERR_UNSUPPORTED, "tile plan: row pairs need complex values and R >= 16");
   cudaStream_t st = m->stream;
@@ -64,7 +68,12 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, TilePlanStore &p
       (e = cudaMemsetAsync(tw.as<uint32_t>() + ntiles, 0, 4, st)) ||
       (e = cudaMemsetAsync(truns.as<uint32_t>() + ntiles, 0, 4, st)))
     return cuda_fail(e, "tile plan: staging");
-  if (R == 8) rc = count_tiles<8>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  if (unit == 2 && R == 64) rc = count_tiles<64, 2>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  else if (unit == 2 && R == 128) rc = count_tiles<128, 2>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  else if (unit == 2 && R == 256) rc = count_tiles<256, 2>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  else if (R == 128 && !cplx) rc = count_tiles<128>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  else if (R == 256 && !cplx) rc = count_tiles<256>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  else if (R == 8) rc = count_tiles<8>(st, m, ntiles, grid, tw, truns, tuniq, flags);
   else if (R == 16) rc = count_tiles<16>(st, m, ntiles, grid, tw, truns, tuniq, flags);
   else if (R == 32) rc = count_tiles<32>(st, m, ntiles, grid, tw, truns, tuniq, flags);
   else if (R == 64) rc = count_tiles<64>(st, m, ntiles, grid, tw, truns, tuniq, flags);
@@ -115,6 +124,14 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, TilePlanStore &p
     if (R == 16) rc = fill_tiles<16, true, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
     else if (R == 32) rc = fill_tiles<32, true, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
     else rc = fill_tiles<64, true, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
+  } else if (unit == 2) {
+    if (R == 64) rc = fill_tiles<64, false, false, 2>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
+    else if (R == 128) rc = fill_tiles<128, false, false, 2>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
+    else rc = fill_tiles<256, false, false, 2>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
+  } else if (R == 128) {
+    rc = fill_tiles<128, false>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
+  } else if (R == 256) {
+    rc = fill_tiles<256, false>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
   } else if (R == 8) rc = TBTKKPM_FILL(8);
   else if (R == 16) rc = TBTKKPM_FILL(16);
   else if (R == 32) rc = TBTKKPM_FILL(32);
@@ -135,6 +152,7 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, TilePlanStore &p
   p.plan.wmax = hf[1];
   p.plan.nruns = nruns;
   p.plan.pairs = pairs ? 1u : 0u;
+  p.plan.unit = unit;
   p.ok = true;
   return TBTKKPM_OK;
 }
@@ -142,15 +160,16 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, TilePlanStore &p
 }  // namespace
 
 // The handle's plan for R-row tiles with real (cplx false) or complex
-// values (pairs: the row-pair plan of complex values), built on first use;
-// *out is null when the matrix has a tile the builder cannot take.
-int tile_plan(tbtkkpm_matrix *m, int R, bool cplx, const TilePlan **out, bool pairs) {
+// values (pairs: the row-pair plan of complex values; unit: columns staged
+// together), built on first use; *out is null when the matrix has a tile the
+// builder cannot take.
+int tile_plan(tbtkkpm_matrix *m, int R, bool cplx, const TilePlan **out, bool pairs, uint32_t unit) {
   *out = nullptr;
-  const int key = (pairs ? 1024 : 0) + 2 * R + (cplx ? 1 : 0);
+  const int key = (int)(unit - 1) * 2048 + (pairs ? 1024 : 0) + 2 * R + (cplx ? 1 : 0);
   auto it = m->plans.find(key);
   if (it == m->plans.end()) {
     TilePlanStore &p = m->plans[key];
-    int rc = build_plan(m, R, cplx, pairs, p);
+    int rc = build_plan(m, R, cplx, pairs, unit, p);
     if (rc) {
       p.release();
       m->plans.erase(key);
