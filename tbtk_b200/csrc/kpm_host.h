@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
+#include <vector>
 
 namespace tbtkkpm {
 
@@ -63,7 +64,8 @@ struct Workspace {
   DevBuf damp;        // [M] damping numerators
   DevBuf out;         // results ([B][E] LDOS)
   DevBuf mu_direct;   // [K][steps+1] directly gathered moments (doubling runs)
-  DevBuf dots;        // [grid][2][Bp] per-block dot products (doubling runs)
+  DevBuf dots;        // [grid][2][Bp] per-block dot products (doubling runs), or the
+                      // warps' sums of an on-chip run
   DevBuf col_out;     // [Bp] output slot of each batch column (doubling runs)
   DevBuf err;         // device flag of a bounded wait that ran out
   DevBuf head, head_jobs, head_res;  // FP64 head of doubling runs (scratch, jobs, results)
@@ -138,6 +140,11 @@ struct tbtkkpm_matrix {
   uint32_t batch_width[3] = {0, 0, 0};
   uint32_t nslices = 0;
   uint64_t chunks = 0;
+  // on-chip recursion (resident.cu), filled on first use: slice_ptr on the
+  // host, its widest slice, groups at once per (kernel shape, shared memory)
+  std::vector<uint32_t> host_slice_ptr;
+  uint32_t widest_slice = 0;
+  std::map<uint64_t, uint32_t> resident_groups;
   tbtkkpm::Workspace ws;
   tbtkkpm::PhaseTimer timer;
   // autotuned step configuration per (kernel class, padded batch width):
@@ -207,6 +214,25 @@ int ldos_sites_terms(tbtkkpm_matrix *m, tbtkkpm_table *t, uint32_t M, const uint
 int moments_pairs(tbtkkpm_matrix *m, const uint32_t *from, uint32_t B, const uint32_t *to,
                   const uint32_t *to_owner, uint32_t K, uint32_t M, double broadening, int precision,
                   bool real64_ok, double *mu_out, double *err_out);
+// Element kinds of the recursion vectors.
+enum VecKind : int { kVecF64C = 0, kVecF64R = 1, kVecC64 = 2, kVecF32 = 3 };
+size_t vec_elem_size(int kind);
+// The on-chip recursion of a batch (kpm_resident.cuh): clusters of `cluster`
+// blocks, each with `cols` sources.  plan_resident leaves ok false where the
+// step kernels serve the batch.
+struct ResidentPlan {
+  bool ok = false, dots = false, reg = false;
+  int kind = 0;
+  uint32_t cluster = 1, cols = 1, groups = 0, warps = 1, spb = 0, chunks = 0, cap = 0;
+  size_t smem = 0;
+};
+struct ResidentArgs;
+constexpr uint32_t kResMaxSlices = 4096;
+int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint32_t *trow,
+                  const uint32_t *tcol, uint32_t T, ResidentPlan &out);
+int launch_resident(cudaStream_t st, int device, const ResidentPlan &p, const ResidentArgs &a);
+void launch_resident_dots(cudaStream_t st, const ResidentPlan &p, uint32_t n0, uint32_t steps, uint32_t B,
+                          const double *part, const uint32_t *col_out, double2 *mu, uint32_t ld, uint32_t M);
 // Lorentz damping numerators a[n] and denominator b (host libm).
 void damping_factors(uint32_t M, double broadening, std::vector<double> &a, double &b);
 // Error estimate of doubled moments against the directly gathered ones.

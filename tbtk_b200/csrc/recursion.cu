@@ -4,6 +4,7 @@
 #include "kpm_kernels.cuh"
 #include "kpm_steps.cuh"
 #include "kpm_prefix.cuh"
+#include "kpm_resident.cuh"
 
 #include <algorithm>
 #include <array>
@@ -248,31 +249,31 @@ ShapeKey shape_key(const tbtkkpm_matrix *m, int cls, uint32_t Bp) {
   return {(uint64_t)m->device, (uint64_t)cls, Bp, m->N, m->nnz};
 }
 
-// The configuration of a batch: a forced entry, the handle's tuned choice
-// for this (class, padded width), this process's choice for a matrix of the
-// same shape, or the default shape with MINB 2.
-const StepEntry *pick_step(const tbtkkpm_matrix *m, int precision, bool dots, uint32_t B,
-                           const StepEntry *force, bool real64) {
-  if (force) return force;
+// The configuration chosen for a batch by set_config or the autotuner: the
+// handle's for this (class, padded width), else this process's for a matrix
+// of the same shape; null where none was.
+const StepEntry *tuned_step(const tbtkkpm_matrix *m, int precision, bool dots, uint32_t B,
+                            bool real64) {
   const bool real = real_mode(m, precision);
-  const int cls = step_class(precision, dots, real);
-  Shape s = shape_for(precision, B, real, dots, m->N);
-  if (real64 && real64_shape_for(B, m->N).bp()) s = real64_shape_for(B, m->N);
-  const int key = real64 ? kClassFP64Real : cls;
-  auto it = m->tuned.find(tune_key(key, s.bp()));
+  const int cls = step_class(precision, dots, real), key = real64 ? kClassFP64Real : cls;
+  const uint32_t Bp = shape_for(precision, B, real, dots, m->N).bp();
+  auto it = m->tuned.find(tune_key(key, Bp));
   if (it != m->tuned.end()) {
     const StepEntry *e = find_step(cls, it->second[0], it->second[1], it->second[2]);
     if (e) return e;
   }
-  {
-    std::lock_guard<std::mutex> lk(g_tuned_mu);
-    auto git = g_tuned.find(shape_key(m, key, s.bp()));
-    if (git != g_tuned.end()) {
-      const StepEntry *e = find_step(cls, git->second[0], git->second[1], git->second[2]);
-      if (e) return e;
-    }
-  }
-  return find_step(cls, s.tpr, s.vpt, s.minb);
+  std::lock_guard<std::mutex> lk(g_tuned_mu);
+  auto git = g_tuned.find(shape_key(m, key, Bp));
+  if (git == g_tuned.end()) return nullptr;
+  return find_step(cls, git->second[0], git->second[1], git->second[2]);
+}
+
+const StepEntry *default_step(const tbtkkpm_matrix *m, int precision, bool dots, uint32_t B,
+                              bool real64) {
+  const bool real = real_mode(m, precision);
+  Shape s = shape_for(precision, B, real, dots, m->N);
+  if (real64 && real64_shape_for(B, m->N).bp()) s = real64_shape_for(B, m->N);
+  return find_step(step_class(precision, dots, real), s.tpr, s.vpt, s.minb);
 }
 
 // A tile-staged entry runs with the matrix's plan for its tile height when
@@ -319,35 +320,51 @@ struct TargetList {
   std::vector<uint32_t> row, col, out;
 };
 
+struct RunOptions {
+  bool use_real64 = false;
+  bool head = true;
+  const StepEntry *force = nullptr;  // this step kernel
+  bool untuned = false;              // not the configuration of set_config or the autotuner
+};
+
 // Runs the recursion of one batch and leaves the undamped moments in ws.mu
 // ([K][M]).  doubling: every source's only target is itself (an LDOS batch);
 // the recursion stops at j_{M/2} and the moments come from the doubling
 // identities, while the directly gathered moments of steps 0..M/2 land in
 // ws.mu_direct ([K][M/2+1]) for the error estimate.  A mixed doubling run
 // on a structurally symmetric matrix takes its first steps in FP64 on the
-// rows they reach (kpm_prefix) unless `head` is false.  use_real64: an FP64
+// rows they reach (kpm_prefix) unless `head` is false.  A small matrix runs
+// its steps on chip in a few launches (plan_resident) unless a step kernel was
+// chosen for the batch.  use_real64: an FP64
 // run of a real matrix takes real vectors; a moment that comes out infinite
 // or NaN then may differ from the complex recursion's, so the caller looks
 // at the moments (or at energy sums over them) and repeats such a run with
 // use_real64 false.
 int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &from,
-              const TargetList &tl, uint32_t K, uint32_t M, bool doubling,
-              const StepEntry *force = nullptr, bool head = true, bool use_real64 = false) {
+              const TargetList &tl, uint32_t K, uint32_t M, bool doubling, const RunOptions &opt) {
   Workspace &ws = m->ws;
   cudaStream_t st = m->stream;
   const uint32_t B = (uint32_t)from.size();
-  const bool real64 = use_real64 && real64_mode(m, precision);
-  const StepEntry *fn = pick_step(m, precision, doubling, B, force, real64);
+  const bool real64 = opt.use_real64 && real64_mode(m, precision);
+  const StepEntry *const force = opt.force;
+  int rc;
+  const StepEntry *fn = force ? force : opt.untuned ? nullptr : tuned_step(m, precision, doubling, B, real64);
+  int kind = real_mode(m, precision) ? kVecF32 : is_mixed(precision) ? kVecC64 : real64 ? kVecF64R : kVecF64C;
+  ResidentPlan res;
+  if (!fn && (rc = plan_resident(m, kind, doubling, B, tl.row.data(), tl.col.data(),
+                                 (uint32_t)tl.row.size(), res))) return rc;
   const TilePlan *plan = nullptr;
-  int rc0 = resolve_tiled(m, precision, doubling, B, force != nullptr, real64, fn, plan);
-  if (rc0) return rc0;
-  if (!fn) return fail(TBTKKPM_ERR_UNSUPPORTED, "no recursion kernel for batch %u", B);
-  const uint32_t Bp = (uint32_t)(fn->tpr * fn->vpt);
+  if (!res.ok) {
+    if (!fn) fn = default_step(m, precision, doubling, B, real64);
+    if ((rc = resolve_tiled(m, precision, doubling, B, force != nullptr, real64, fn, plan))) return rc;
+    if (!fn) return fail(TBTKKPM_ERR_UNSUPPORTED, "no recursion kernel for batch %u", B);
+    kind = fn->cls == kClassFP64 ? kVecF64C : fn->cls == kClassFP64Real ? kVecF64R
+           : fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots ? kVecF32 : kVecC64;
+  }
+  const uint32_t Bp = res.ok ? res.groups * res.cols : (uint32_t)(fn->tpr * fn->vpt);
   if (Bp < B) return fail(TBTKKPM_ERR_ARGUMENT, "configuration of %u columns for %u sources", Bp, B);
-  const bool real = fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots;
-  const size_t esize = real ? sizeof(float)
-                       : is_mixed(precision) ? sizeof(float2)
-                       : fn->cls == kClassFP64Real ? sizeof(double) : sizeof(double2);
+  const bool real = kind == kVecF32;
+  const size_t esize = vec_elem_size(kind);
   // rows of 8 bytes are staged two at a time: one padding row for an odd N
   const size_t vbytes = (size_t)m->N * Bp * esize + (Bp * esize < 16 ? 16 : 0);
   const size_t words = ((size_t)m->N + 31) / 32;
@@ -355,7 +372,13 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
   const uint32_t steps = doubling ? M / 2 : (M >= 2 ? M - 1 : 0);  // last j index computed
   const uint32_t ld_direct = doubling ? steps + 1 : M;
   const unsigned max_grid = (unsigned)sm_count(m->device) * 8;
-  int rc;
+  // an on-chip run takes its steps in launches whose doubling sums fit 64 MB
+  const size_t step_part = 16 * (size_t)res.groups * res.cols * res.cluster;
+  const uint32_t per_launch =
+      doubling ? (uint32_t)std::max<size_t>(32, std::min<size_t>(steps, ((size_t)64 << 20) / std::max<size_t>(step_part, 1)))
+               : 4096;
+  const size_t dots_bytes =
+      res.ok ? step_part * std::min(per_launch, std::max(steps, 1u)) : sizeof(double2) * 2 * (size_t)Bp * max_grid;
   if ((rc = ws.vec[0].reserve(vbytes)) || (rc = ws.vec[1].reserve(vbytes)) ||
       (rc = ws.bitmap.reserve(4 * words)) || (rc = ws.tgt.reserve(12 * std::max(T, 1u))) ||
       (rc = ws.from.reserve(4 * std::max(B, 1u))) || (rc = ws.err.reserve(16)) ||
@@ -363,7 +386,7 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
     return rc;
   if (doubling &&
       ((rc = ws.mu_direct.reserve(sizeof(double2) * (size_t)std::max(K, 1u) * ld_direct)) ||
-       (rc = ws.dots.reserve(sizeof(double2) * 2 * (size_t)Bp * max_grid)) ||
+       (rc = ws.dots.reserve(dots_bytes)) ||
        (rc = ws.col_out.reserve(4 * (size_t)Bp))))
     return rc;
   std::vector<uint32_t> bitmap(words, 0u);
@@ -400,7 +423,7 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
   // FP64 head: j_0 .. j_q of every source on its ball, q common to the batch
   uint32_t q = 0;
   const uint32_t want = std::min(m->head_steps, steps >= 1 ? steps - 1 : 0u);
-  if (head && doubling && is_mixed(precision) && m->pattern_symmetric && want >= 2) {
+  if (opt.head && doubling && is_mixed(precision) && m->pattern_symmetric && want >= 2) {
     std::vector<uint32_t> slot(B, kPad);
     for (uint32_t i = 0; i < T; i++) slot[tl.col[i]] = tl.out[i];
     if (std::find(slot.begin(), slot.end(), kPad) != slot.end())
@@ -456,7 +479,7 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
   } else if (real) {
     kpm_init_sources_real<<<ib, 256, 0, st>>>(B, Bp, ws.from.as<uint32_t>(), ws.vec[0].as<float>(),
                                               tg);
-  } else if (fn->cls == kClassFP64Real) {
+  } else if (kind == kVecF64R) {
     kpm_init_sources_real<<<ib, 256, 0, st>>>(B, Bp, ws.from.as<uint32_t>(), ws.vec[0].as<double>(),
                                               tg);
   } else if (is_mixed(precision)) {
@@ -476,8 +499,34 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
   m->timer.mark(st, 0);
   m->timer.pending = m->timer.enabled;
   m->timer.pending_steps = steps - q;
-  count_launches((q > 0 ? 0 : 1) + (uint64_t)(steps - q) * (doubling ? 2 : 1));
-  for (uint32_t n = q + 1; n <= steps; n++) {
+  count_launches(q > 0 ? 0 : 1);
+  for (uint32_t n = q + 1; res.ok && n <= steps; n += per_launch) {
+    ResidentArgs r{};
+    r.A = a.A;
+    r.spb = res.spb;
+    r.chunks = res.chunks;
+    r.cap = res.cap;
+    r.Bp = Bp;
+    r.x = cur;
+    r.y = prev;
+    r.n0 = n;
+    r.n1 = std::min(steps, n + per_launch - 1);
+    r.keep = r.n1 < steps;
+    r.tg = tg;
+    r.part = doubling ? ws.dots.as<double>() : nullptr;
+    if ((rc = launch_resident(st, m->device, res, r))) return rc;
+    if (!doubling) continue;
+    if (n == 1) {
+      e = cudaMemcpy2DAsync(ws.mu.ptr, sizeof(double2) * M, ws.mu_direct.ptr,
+                            sizeof(double2) * ld_direct, sizeof(double2) * std::min(M, 2u),
+                            K, cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return cuda_fail(e, "recursion: seed moments");
+    }
+    launch_resident_dots(st, res, n, r.n1 - n + 1, B, ws.dots.as<double>(), ws.col_out.as<uint32_t>(),
+                         ws.mu.as<double2>(), M, M);
+  }
+  if (!res.ok) count_launches((uint64_t)(steps - q) * (doubling ? 2 : 1));
+  for (uint32_t n = q + 1; !res.ok && n <= steps; n++) {
     a.x = cur;
     a.y = prev;
     a.n_out = n;
@@ -653,7 +702,7 @@ static int moments_host(tbtkkpm_matrix *m, const uint32_t *from, uint32_t B, con
     const uint32_t Kb = (uint32_t)global_k.size();
     mu_host.resize((size_t)Kb * M);
     for (bool real64 = real64_ok;; real64 = false) {
-      int rc = run_batch(m, precision, fr, tl, Kb, M, false, nullptr, true, real64);
+      int rc = run_batch(m, precision, fr, tl, Kb, M, false, {real64});
       if (rc) return rc;
       m->timer.mark(m->stream, 2);
       m->timer.mark(m->stream, 3);
@@ -1114,7 +1163,7 @@ int tbtkkpm::ldos_sites_terms(tbtkkpm_matrix *m, tbtkkpm_table *t, uint32_t M, c
     }
     const uint32_t ld = M / 2 + 1;
     for (bool real64 = true;; real64 = false) {
-      if ((rc = run_batch(m, precision, fr, tl, nb, M, doubling, nullptr, true, real64))) return rc;
+      if ((rc = run_batch(m, precision, fr, tl, nb, M, doubling, {real64}))) return rc;
       if (doubling && err_out) {
         // undamped moments for the estimate
         mu_h.resize((size_t)nb * M);
@@ -1173,7 +1222,8 @@ int tbtkkpm::ldos_sites_terms(tbtkkpm_matrix *m, tbtkkpm_table *t, uint32_t M, c
 // Times every compiled step configuration whose padded width serves B
 // sources on this matrix (probe_steps steps each, best of two runs, CUDA
 // events on the handle's stream around the steps) and keeps the fastest for
-// later batches of that width on this handle.
+// later batches of that width on this handle, unless such batches run on
+// chip and that is faster still.
 extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precision, int ldos,
                                        uint32_t probe_steps, int *tpr, int *vpt, int *minb,
                                        double *ms_per_step) {
@@ -1210,33 +1260,37 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   const bool real64 = ldos && real64_mode(m, precision);
   const StepEntry *best = nullptr, *best_cplx = nullptr;
   double best_ms = 0, best_cplx_ms = 0;
-  for (int i = 0; i < n; i++) {
-    if ((uint32_t)(t[i].tpr * t[i].vpt) != Bp) continue;
-    if (t[i].cls == kClassFP64Real && !real64) continue;
-    double ms = 0;
-    bool skip = false;
+  // best of two runs of a step kernel (null: the untuned default) in ms per
+  // step, or -1 for a tile-staged step whose ring does not fit this matrix
+  auto time_step = [&](const StepEntry *e, double &ms) -> int {
     for (int rep = 0; rep < 2; rep++) {
       m->timer.recursion_ms = 0;
-      if ((rc = run_batch(m, precision, fr, tl, B, M, doubling, &t[i], false, real64))) {
-        // a tile-staged step whose ring does not fit this matrix
-        if (rc == TBTKKPM_ERR_UNSUPPORTED && is_tiled_variant(t[i].minb)) {
-          rc = TBTKKPM_OK;
-          skip = true;
-        }
-        break;
+      RunOptions opt;
+      opt.use_real64 = real64;
+      opt.head = false;
+      opt.force = e;
+      opt.untuned = true;
+      int r = run_batch(m, precision, fr, tl, B, M, doubling, opt);
+      if (r == TBTKKPM_ERR_UNSUPPORTED && e && is_tiled_variant(e->minb)) {
+        ms = -1;
+        return TBTKKPM_OK;
       }
-      cudaError_t e = cudaStreamSynchronize(m->stream);
-      if (e != cudaSuccess) {
-        rc = cuda_fail(e, "matrix_autotune");
-        break;
-      }
+      if (r) return r;
+      cudaError_t err = cudaStreamSynchronize(m->stream);
+      if (err != cudaSuccess) return cuda_fail(err, "matrix_autotune");
       m->timer.collect();
-      if ((rc = check_device_flag(m))) break;
+      if ((r = check_device_flag(m))) return r;
       const double v = m->timer.recursion_ms / probe_steps;
       ms = rep == 0 ? v : std::min(ms, v);
     }
-    if (rc) break;
-    if (skip) continue;
+    return TBTKKPM_OK;
+  };
+  for (int i = 0; i < n && !rc; i++) {
+    if ((uint32_t)(t[i].tpr * t[i].vpt) != Bp) continue;
+    if (t[i].cls == kClassFP64Real && !real64) continue;
+    double ms = 0;
+    if ((rc = time_step(&t[i], ms))) break;
+    if (ms < 0) continue;
     if (!best || ms < best_ms) {
       best = &t[i];
       best_ms = ms;
@@ -1245,6 +1299,17 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
       best_cplx = &t[i];
       best_cplx_ms = ms;
     }
+  }
+  // The default of a batch that runs on chip stays where it beats every step
+  // kernel: no configuration is recorded then.
+  bool keep_default = false;
+  ResidentPlan res;
+  const int kind = real ? kVecF32 : is_mixed(precision) ? kVecC64 : real64 ? kVecF64R : kVecF64C;
+  if (!rc) rc = plan_resident(m, kind, doubling, B, tl.row.data(), tl.col.data(), B, res);
+  if (!rc && res.ok) {
+    double ms = 0;
+    rc = time_step(nullptr, ms);
+    keep_default = !rc && best && ms < best_ms;
   }
   const bool created = saved.ev[0] == nullptr;
   if (created) m->timer.destroy();
@@ -1259,8 +1324,13 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   if (!best) return fail(TBTKKPM_ERR_UNSUPPORTED, "matrix_autotune: no configuration for %u", B);
   auto keep = [&](int key, const StepEntry *e) {
     if (!e) return;
-    m->tuned[tune_key(key, Bp)] = {e->tpr, e->vpt, e->minb};
     std::lock_guard<std::mutex> lk(g_tuned_mu);
+    if (keep_default) {
+      m->tuned.erase(tune_key(key, Bp));
+      g_tuned.erase(shape_key(m, key, Bp));
+      return;
+    }
+    m->tuned[tune_key(key, Bp)] = {e->tpr, e->vpt, e->minb};
     g_tuned[shape_key(m, key, Bp)] = {e->tpr, e->vpt, e->minb};
   };
   if (real64) keep(kClassFP64Real, best);
