@@ -179,8 +179,10 @@ TILED_REAL = {
     (32, 4): _variants([(32, 8, 2), (64, 16, 1), (16, 8, 2)], [0, 51]),
     (32, 8): _variants([(16, 8, 2), (32, 16, 1), (16, 16, 1)], [0, 51]),
     # 4-8 sources: small blocks, several per SM
-    (1, 4): _variants([(64, 2, 8), (64, 2, 6)], [0, 51]),
-    (1, 8): _variants([(64, 2, 8), (64, 2, 6)], [0, 51]),
+    (1, 1): _variants([(256, 8, 3), (256, 8, 2), (128, 4, 6), (64, 2, 8)], [0]),
+    (1, 2): _variants([(256, 8, 3), (256, 8, 2), (128, 4, 6), (64, 2, 8)], [0]),
+    (1, 4): _variants([(64, 2, 8), (64, 2, 6)], [0, 51]) + _variants([(256, 8, 2), (128, 4, 6), (128, 4, 4)], [0]),
+    (1, 8): _variants([(64, 2, 8), (64, 2, 6), (128, 4, 4)], [0, 51]),
     (2, 4): _variants([(64, 4, 6), (64, 4, 4)], [0, 51]),
     (2, 8): _variants([(64, 4, 4), (64, 4, 6)], [0, 51]),
 }
@@ -205,9 +207,10 @@ TILED_CPLX = {
     (64, 2): _variants([(16, 16, 1)], [100, 151]),
     (8, 2): _variants([(32, 8, 2), (16, 8, 2)], [0, 60]),
     # 2-8 sources: small blocks, several per SM
-    (1, 2): _variants([(64, 2, 8), (64, 2, 6)], [0, 60]),
-    (1, 4): _variants([(64, 2, 8)], [0, 60]),
-    (2, 2): _variants([(64, 4, 6)], [0, 60]),
+    (1, 1): _variants([(64, 2, 8), (64, 2, 6), (128, 4, 4)], [0]),
+    (1, 2): _variants([(64, 2, 8), (64, 2, 6)], [0, 60]) + _variants([(64, 2, 4)], [0]),
+    (1, 4): _variants([(64, 2, 8)], [0, 60]) + _variants([(128, 4, 3)], [0]),
+    (2, 2): _variants([(64, 4, 6)], [0, 60]) + _variants([(64, 4, 4)], [0]),
     (2, 4): _variants([(64, 4, 4), (64, 4, 6)], [0, 60]),
     (4, 2): _variants([(64, 8, 4)], [0, 60]),
 }
@@ -218,9 +221,9 @@ TILED_CPLX = {
 # warps, blocks per SM).  Rows of 16-byte values: B = 16 / 32 / 64 / 128
 # take 256 B / 512 B / 1 KB / 2 KB per row.
 TILED_FP64 = {
-    (1, 1): [(64, 2, 8), (64, 2, 6), (32, 1, 8), (64, 2, 4)],
-    (2, 1): [(64, 4, 6), (64, 4, 4), (32, 2, 8)],
-    (4, 1): [(64, 8, 4), (64, 8, 2), (32, 4, 6)],
+    (1, 1): [(64, 2, 8), (64, 2, 6), (64, 2, 4), (128, 4, 4)],
+    (2, 1): [(64, 4, 6), (64, 4, 4), (128, 8, 3)],
+    (4, 1): [(64, 8, 4), (64, 8, 3), (64, 8, 2), (32, 4, 6)],
     (8, 1): [(64, 16, 2), (32, 8, 4), (64, 8, 3)],
     (16, 1): [(32, 8, 2), (64, 16, 1)],
     (32, 1): [(32, 8, 2), (16, 8, 2), (64, 16, 1)],

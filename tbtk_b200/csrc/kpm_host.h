@@ -87,7 +87,7 @@ struct TilePlan {
   uint32_t umax, wmax;     // most distinct outside columns / entries per row of a tile
   uint32_t nruns;          // runs of all tiles
   uint32_t pairs;          // row-pair plan: entries of [w][R/2] row pairs, two values each
-  uint32_t unit;           // columns staged together (2: for vector rows of 8 bytes)
+  uint32_t unit;           // columns staged together (1 or 4)
 };
 
 // Byte layout of one shared-memory ring stage of a tile-staged step
@@ -248,9 +248,9 @@ double ldos_error_estimate(double moment_err, double wmax, const double *row, ui
 void doubling_error(const std::vector<double2> &mu, const std::vector<double2> &direct,
                     uint32_t K, uint32_t M, uint32_t ld, double *err);
 // The matrix's gather plan for R-row tiles (real or complex values; pairs:
-// the row-pair plan of complex values, R >= 16; unit 2: columns staged in
-// pairs, real values and R = 64), built on first use; *out is null when some
-// tile is too large for the builder.
+// the row-pair plan of complex values, R >= 16; unit: 1 or 4 columns staged
+// together), built on first use; *out is null when some tile is too
+// large for the builder.
 int tile_plan(tbtkkpm_matrix *m, int R, bool cplx, const TilePlan **out, bool pairs = false,
               uint32_t unit = 1);
 

@@ -56,6 +56,13 @@ __device__ __forceinline__ double2 cmac(double2 acc, double2 v, double2 x) {
   }
 }
 
+// ---------------------------------------------------------------- dependent launches
+// A step launched with programmatic stream serialization starts while the
+// step before it drains; pdl_wait returns when that one has ended and its
+// writes are visible (both do nothing in a kernel launched without it).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------- vector packs
 // The VPT complex values a thread owns in one row of a batch, as raw loads:
 // complex128 as double2 each; complex64 as float2 (VPT = 1) or float4 pairs.
@@ -558,13 +565,16 @@ kpm_step(Sell A, uint32_t Bp, const V *__restrict__ x, V *__restrict__ y, Target
 // mu_{2m} = 2<j_m|j_m> - mu_0 and mu_{2m-1} = 2<j_m|j_{m-1}> - mu_1 for the
 // step that produced j_m.  One block per batch column sums the partials in
 // a fixed tree order (deterministic).  col_out[c] is the output slot of
-// batch column c (or kPad).
+// batch column c (or kPad).  blockIdx.y counts steps from m0, whose partials
+// lie `stride` values apart: one launch serves many steps, since a launch
+// after every step held up the next one by 4-6 us.
 constexpr int kFinalizeBlock = 128;
 static __global__ void __launch_bounds__(kFinalizeBlock)
-kpm_dots_finalize(uint32_t Bp, uint32_t nblocks, const double2 *__restrict__ dots,
+kpm_dots_finalize(uint32_t Bp, uint32_t nblocks, const double2 *__restrict__ dots, uint64_t stride,
                   const uint32_t *__restrict__ col_out, double2 *mu, uint32_t ld, uint32_t M,
-                  uint32_t m) {
-  const uint32_t c = blockIdx.x;
+                  uint32_t m0) {
+  const uint32_t c = blockIdx.x, m = m0 + blockIdx.y;
+  dots += blockIdx.y * stride;
   const uint32_t slot = col_out[c];
   if (slot == kPad) return;
   __shared__ double ra[kFinalizeBlock], rbx[kFinalizeBlock], rby[kFinalizeBlock];

@@ -186,10 +186,32 @@ void launch_async(cudaStream_t st, int device, unsigned max_grid, const StepArgs
 // warps, BPS blocks per SM).
 constexpr int kTiledVariant = 100000;
 constexpr int kTiledReal64 = 200;
+// Columns staged together: the copies move multiples of 16 bytes, so rows of
+// 8 and 4 bytes go two and four at a time.
+constexpr uint32_t tiled_unit(uint32_t rowbytes) { return rowbytes >= 16 ? 1 : 16 / rowbytes; }
 inline bool is_tiled_variant(int v) { return v >= kTiledVariant; }
 inline int tiled_rows(int v) { return ((v - kTiledVariant) % 1000000) / 1000; }
 inline bool tiled_pairs(int v) { return (v - kTiledVariant) / 1000000 / 100 == 1; }
 inline int tiled_bps(int v) { return v % 10; }
+inline int tiled_warps(int v) { return (v - kTiledVariant) % 1000 / 10; }
+
+// Launches with programmatic stream serialization: the kernel's blocks may
+// start while the kernel before it drains (pdl_wait).
+template <typename... P, typename... A>
+void launch_dependent(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                      A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 
 template <bool CPLX, int TPR, int VPT, int R, int CW, int BPS, bool FIRST, bool DOTS, int CV,
           bool F64 = false>
@@ -199,10 +221,9 @@ void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs
   using Val = typename TiledTypes<CPLX, F64>::Val;
   auto kern = kpm_step_tiled<CPLX, TPR, VPT, R, CW, BPS, FIRST, DOTS, CV, F64>;
   *grid = 0;
-  // columns staged together: two for rows of 8 bytes (the copies' 16-byte rule)
-  constexpr uint32_t unit = TPR * VPT * sizeof(E) < 16 ? 2u : 1u;
+  constexpr uint32_t unit = tiled_unit(TPR * VPT * sizeof(E));
   if (!a.plan || a.plan->R != (uint32_t)R || a.plan->pairs != (CV >= 100 ? 1u : 0u) ||
-      a.plan->unit != unit)
+      a.plan->unit % unit)
     return;
   const TilePlan &p = *a.plan;
   const TiledLayout ly =
@@ -218,12 +239,17 @@ void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs
   if (max_grid) g = std::min<uint64_t>(g, max_grid);
   g = std::max<uint64_t>(g, 1);
   *grid = (unsigned)g;
-  // the ring holds the block's dot-product reduction at the end (2 doubles
-  // per consumer thread)
-  const uint32_t smem = kTiledHeader + std::max(ly.stages * ly.stage_bytes, 32u * CW * 16u);
-  kern<<<(unsigned)g, 32 * (CW + 1), smem, st>>>(
-      p, ly, a.Bp, static_cast<const E *>(a.x), static_cast<E *>(a.y), a.tg, a.n_out, a.dots,
-      a.err, a.wait_limit);
+  // The ring holds the block's dot-product reduction at the end (2 doubles
+  // per consumer thread).  A full grid takes its whole share of the SM, so
+  // that never more than BPS blocks fit one: blocks placed while the step
+  // before drains would else pile up on the SMs that end first (10% slower
+  // at 4 FP64 sources on the 1024^2 lattice).
+  static_assert(tiled_budget(BPS) >= kTiledHeader + 32u * CW * 16u, "reduction scratch");
+  const uint32_t need = kTiledHeader + std::max(ly.stages * ly.stage_bytes, 32u * CW * 16u);
+  const uint32_t smem = g == (uint64_t)BPS * sm_count(device) ? tiled_budget(BPS) : need;
+  launch_dependent(kern, (unsigned)g, 32 * (CW + 1), smem, st, p, ly, a.Bp,
+                   static_cast<const E *>(a.x), static_cast<E *>(a.y), a.tg, a.n_out, a.dots, a.err,
+                   a.wait_limit);
 }
 
 #define TBTKKPM_TILED_ENTRY(CLS, CPLX, T, P, D, R, CW, BPS, CV)                     \

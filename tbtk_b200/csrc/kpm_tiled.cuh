@@ -224,6 +224,11 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
+  // the next step's blocks may take this one's place as it drains; they read
+  // vectors only after pdl_wait, and only by bulk copies (no L1 line of an
+  // overlapping step can be stale)
+  pdl_trigger();
+  if (warp != 0) pdl_wait();
 
   const int ct = threadIdx.x - 32;
   const int sub = ct >= 0 ? ct % TPR : 0, grp = ct >= 0 ? ct / TPR : 0;
@@ -259,8 +264,8 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
       const uint32_t r0 = t * R, Rt = min((uint32_t)R, P.N - r0);
       // pair entries carry two values each: w * R values either way
       const uint32_t ebytes = w * R * (uint32_t)sizeof(Val), sbytes = w * EW * 2u;
-      // rows of 8 bytes: the last tile's own rows may be odd, its copies take
-      // the buffer's padding row too (runs come in whole plan units)
+      // rows of 4 or 8 bytes: the last tile's own rows may not fill 16 bytes,
+      // its copies take the buffer's padding too (runs come in whole units)
       const uint32_t obytes = rowbytes < 16u ? align_up(Rt * rowbytes, 16) : Rt * rowbytes;
       const uint32_t bytes = ebytes + sbytes + nuniq * rowbytes + (FIRST ? 1u : 2u) * obytes;
       if (lane == 0) mbar_expect_tx(&full[s], bytes);
@@ -270,6 +275,10 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
         if (lane == 0)
           bulk_load(st, static_cast<const Val *>(P.eval) + e0 * (PAIR ? 2 : 1), ebytes, &full[s]);
         if (lane == 1) bulk_load(st + LY.off_slots, P.eslot + e0, sbytes, &full[s]);
+      }
+      if (i == 0) {  // the plan does not depend on the step before, the vectors do
+        pdl_wait();
+        asm volatile("fence.proxy.async.global;" ::: "memory");
       }
       if (lane == 2) bulk_load(st + LY.off_xs, x + (uint64_t)r0 * Bp, obytes, &full[s]);
       if (!FIRST && lane == 3)
@@ -654,8 +663,8 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
 // the runs of consecutive ones counted (k_plan_count) or listed
 // (k_plan_fill).  A tile with more than kPlanCap entries sets *bad.
 
-// UNIT is the number of columns staged together: 1, or 2 for vector rows of
-// 8 bytes, whose copies would otherwise break the 16-byte rule.  A unit is
+// UNIT is the number of columns staged together: 1, or 2 or 4 for vector rows
+// of 8 or 4 bytes, whose copies would otherwise break the 16-byte rule.  A unit is
 // the columns [UNIT*i, UNIT*(i + 1)); runs and slots are in columns.
 
 // Loads the units of the tile's outside columns (each by its first column)

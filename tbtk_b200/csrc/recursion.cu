@@ -115,17 +115,14 @@ constexpr int tiled(int cv, int rows, int cw, int bps) {
 // FP64 steps on real vectors (kClassFP64Real).
 constexpr int tiled64r(int rows, int cw, int bps) { return tiled(kTiledReal64, rows, cw, bps); }
 
-// Default FP64 shape of a real matrix, {0, 0} where the complex steps stay.
-// us per step on the 2048^2 lattice (best of the complex steps in brackets)
-// for B = 1 / 2 / 4 / 8: 94 (170) / 122 (223) / 184 (345) / 317 (667), for
-// B = 16 / 32 / 64 / 128: 532 (1385) / 967 (2138) / 2047 (4207) / 4081
-// (8386); at 131k rows 8.2 (9.1) / 10 (14) / 13 (27) / 18 (41) / 41 (73) / 73
-// (141) for B = 4 ... 128, at 16k rows 6.2 (8.2) / 8.2 (10.3) / 10.3 (14.2)
-// for B = 16 / 32 / 64 and even below.  A single source is faster on the
-// complex thread per row up to 65k rows (5.1 against 6.2 us) and even at
-// 131k.
-Shape real64_shape_for(uint32_t B, uint32_t N) {
-  if (B <= 1) return N <= (1u << 17) ? Shape{0, 0} : Shape{1, 1, tiled64r(256, 8, 3)};
+// Default FP64 shape of a real matrix.  us per step on the 2048^2 lattice
+// (best of the complex steps in brackets) for B = 1 / 2 / 4 / 8: 94 (170) /
+// 122 (223) / 184 (345) / 317 (667), for B = 16 / 32 / 64 / 128: 532 (1385) /
+// 967 (2138) / 2047 (4207) / 4081 (8386); on 181^2 sites, with dependent
+// launches: 2.8 (3.4) / 3.8 (4.7) / 4.7 (7.5) / 7.3 (13) / 9.3 (18) / 19 (38) /
+// 38 (73) for B = 2 ... 128.
+Shape real64_shape_for(uint32_t B) {
+  if (B <= 1) return {1, 1, tiled64r(256, 8, 3)};
   if (B <= 2) return {1, 2, tiled64r(256, 8, 3)};
   if (B <= 4) return {1, 4, tiled64r(64, 2, 8)};
   if (B <= 8) return {4, 2, tiled64r(64, 8, 4)};
@@ -135,71 +132,63 @@ Shape real64_shape_for(uint32_t B, uint32_t N) {
   return {16, 8, tiled64r(8, 8, 2)};
 }
 
-// Default shape of a batch.  At mixed precision from 32 sources on (from 16
-// for complex vectors) the tile-staged steps are the defaults: ms per step
-// measured on the 2048^2 lattice (real float vectors, doubling dots) for
-// B = 32 / 64 / 128 / 256: 1.05 / 1.43 / 3.01 / 5.71 against 1.82 / 2.90 /
-// 4.79 / 11.8 for the register-staged defaults, and on the 1024^2 Rashba
-// lattice (complex64) for B = 16 / 32 / 64 / 128 / 256: 0.38 / 0.55 / 1.09 /
-// 2.14 / 4.27 against 1.06 / 1.25 / 1.94 / 3.33 / 8.28.  Without the dots
-// (directly gathered moments) the real B = 64 step takes 1.29 ms (0.84 of
-// the measured copy bandwidth).  A matrix whose tiles do not fit the ring
-// falls back to register_shape_for.
+// Default shape of a batch.  At mixed precision ms per step measured on the
+// 2048^2 lattice (real float vectors, doubling dots) for B = 32 / 64 / 128 /
+// 256: 1.05 / 1.43 / 3.01 / 5.71 against 1.82 / 2.90 / 4.79 / 11.8 for the
+// register-staged defaults, and on the 1024^2 Rashba lattice (complex64) for
+// B = 16 / 32 / 64 / 128 / 256: 0.38 / 0.55 / 1.09 / 2.14 / 4.27 against 1.06 /
+// 1.25 / 1.94 / 3.33 / 8.28.  Without the dots (directly gathered moments) the
+// real B = 64 step takes 1.29 ms (0.84 of the measured copy bandwidth).  A
+// matrix whose tiles do not fit a shape's ring takes the next one that does
+// (resolve_tiled).
 // N: the matrix's rows (0: large).
 Shape shape_for(int precision, uint32_t B, bool real = false, bool dots = false, uint32_t N = 0) {
   if (!is_mixed(precision)) {
     // FP64 (complex128 vectors) on the 2048^2 lattice, ms per step for
-    // B = 1 / 2 / 4 / 8 / 16: 0.171 / 0.224 / 0.346 / 0.669 / 1.38
-    // tile-staged against 0.278 / 0.504 / 0.924 / 2.49 / 4.50
+    // B = 1 / 2 / 4 / 8 / 16: 0.166 / 0.219 / 0.339 / 0.669 / 1.38
+    // tile-staged against 0.278 / 0.503 / 0.924 / 2.49 / 4.50
     // register-staged, and for B = 32 / 64 / 128: 2.12 / 4.12 / 8.32
     // (0.96-0.99 of the measured copy bandwidth) against 5.28 / 6.79 / 18.9.
-    // Below 2^17 rows a single source is faster register-staged (4.4 against
-    // 5.2 us per step at 32k rows); at 32 sources tile staging is as fast or
-    // faster from 2k rows on.
-    const bool big = N == 0 || N > (1u << 17);
-    if (B <= 1 && big) return {1, 1, tiled(0, 64, 2, 8)};
-    if (B == 2 && big) return {2, 1, tiled(0, 64, 4, 6)};
-    if (B > 2 && B <= 4 && big) return {4, 1, tiled(0, 64, 8, 4)};
-    if (B > 4 && B <= 8 && big) return {8, 1, tiled(0, 64, 16, 2)};
-    if (B > 8 && B <= 16 && big) return {16, 1, tiled(0, 32, 8, 2)};
-    if (B > 16 && B <= 32) return {16, 2, tiled(0, 16, 8, 2)};
-    if (B > 32 && B <= 64) return {16, 4, tiled(0, 8, 8, 2)};
-    if (B > 64) return {32, 4, tiled(0, 8, 16, 1)};
+    // Dependent launches make tile staging the faster at every size: 181^2
+    // sites, B = 1 / 2 / 4: 2.9 / 3.4 / 4.6 us against 4.6 / 8.2 / 10.3.
+    if (B <= 1) return {1, 1, tiled(0, 64, 2, 8)};
+    if (B == 2) return {2, 1, tiled(0, 64, 4, 6)};
+    if (B <= 4) return {4, 1, tiled(0, 64, 8, 4)};
+    if (B <= 8) return {8, 1, tiled(0, 64, 16, 2)};
+    if (B <= 16) return {16, 1, tiled(0, 32, 8, 2)};
+    if (B <= 32) return {16, 2, tiled(0, 16, 8, 2)};
+    if (B <= 64) return {16, 4, tiled(0, 8, 8, 2)};
+    return {32, 4, tiled(0, 8, 16, 1)};
   }
-  if (is_mixed(precision)) {
-    // 2-8 sources (rows of 16-64 bytes): small tile-staged blocks, several
-    // per SM; doubling LDOS, ms per step for real B = 4 / 8 on the 2048^2
-    // lattice 0.167 / 0.237 against 0.347 / 0.505 register-staged (0.0146 /
-    // 0.0165 against 0.0186 / 0.0234 at 131k rows), complex B = 2 / 4 / 8 on
-    // the 1024^2 Rashba lattice 0.079 / 0.099 / 0.156 against 0.138 / 0.170
-    // / 0.383; real B = 16: 0.408 against 0.836 (0.0207 against 0.0267 at
-    // 131k rows).  At 2k rows real B = 8 / 16 steps are faster with a
-    // register-staged thread per row (10.3 against 12.4 / 13.4 us; about
-    // even at 32k rows).
-    const bool tiny = N != 0 && N <= (1u << 14);
-    if (real) {
-      if (B > 2 && B <= 4) return {1, 4, tiled(0, 64, 2, 8)};
-      if (B > 4 && B <= 8 && !tiny) return {1, 8, tiled(0, 64, 2, 8)};
-      if (B > 8 && B <= 16 && !tiny) return {2, 8, tiled(51, 64, 4, 4)};
-    } else {
-      if (B == 2) return {1, 2, tiled(0, 64, 2, 6)};
-      if (B > 2 && B <= 4) return {2, 2, tiled(0, 64, 4, 6)};
-      if (B > 4 && B <= 8) return {2, 4, tiled(0, 64, 4, 4)};
-    }
-    if (real) {
-      if (B > 16 && B <= 32) return {8, 4, tiled(0, 64, 16, 1)};
-      if (B > 32 && B <= 64) return {8, 8, tiled(51, 64, 16, 1)};
-      if (B > 64 && B <= 128) return {16, 8, tiled(51, 16, 8, 2)};
-      if (B > 128) return {32, 8, tiled(51, 16, 16, 1)};
-    } else {
-      if (B > 8 && B <= 16) return {8, 2, tiled(0, 32, 8, 2)};
-      if (B > 16 && B <= 32) return {8, 4, tiled(0, 32, 8, 2)};
-      if (B > 32 && B <= 64) return {16, 4, tiled(0, 16, 8, 2)};
-      if (B > 64 && B <= 128) return {32, 4, tiled(0, 16, 16, 1)};
-      if (B > 128) return {64, 4, tiled(0, 8, 16, 1)};
-    }
+  // Small batches: rows of 4-64 bytes, small tile-staged blocks, several per
+  // SM.  Doubling LDOS, us per step: real B = 1 / 2 / 4 / 8 on 1024^2 sites
+  // 24 / 29 / 37 / 59 against 60 / 64 / 95 / 150 register-staged, on 181^2
+  // 4.0 / 5.4 / 5.7 / 6.3 against 6.3 / 8.4 / 10 / 16; complex B = 1 / 2 / 4 /
+  // 8 on the 512^2 Rashba lattice 14 / 20 / 25 / 40 against 31 / 39 / 46 /
+  // 100.  Below 2^18 rows four and eight real sources are faster in 64-row
+  // tiles (5.7 and 6.3 us against 6.7 and 8.4), above in 128-row ones (37 and
+  // 59 us against 44 and 62 at 2^21 rows).
+  const bool small = N != 0 && N <= (1u << 18);
+  if (real) {
+    if (B <= 1) return {1, 1, tiled(0, 256, 8, 3)};
+    if (B <= 2) return {1, 2, tiled(0, 256, 8, 3)};
+    if (B <= 4) return small ? Shape{1, 4, tiled(0, 64, 2, 8)} : Shape{1, 4, tiled(0, 128, 4, 6)};
+    if (B <= 8) return small ? Shape{2, 4, tiled(0, 64, 4, 4)} : Shape{1, 8, tiled(51, 128, 4, 4)};
+    if (B <= 16) return {2, 8, tiled(51, 64, 4, 4)};
+    if (B <= 32) return {8, 4, tiled(0, 64, 16, 1)};
+    if (B <= 64) return {8, 8, tiled(51, 64, 16, 1)};
+    if (B <= 128) return {16, 8, tiled(51, 16, 8, 2)};
+    return {32, 8, tiled(51, 16, 16, 1)};
   }
-  return register_shape_for(precision, B, real, dots);
+  if (B <= 1) return {1, 1, tiled(0, 64, 2, 8)};
+  if (B == 2) return {1, 2, tiled(0, 64, 2, 6)};
+  if (B <= 4) return {2, 2, tiled(0, 64, 4, 6)};
+  if (B <= 8) return {2, 4, tiled(0, 64, 4, 4)};
+  if (B <= 16) return {8, 2, tiled(0, 32, 8, 2)};
+  if (B <= 32) return {8, 4, tiled(0, 32, 8, 2)};
+  if (B <= 64) return {16, 4, tiled(0, 16, 8, 2)};
+  if (B <= 128) return {32, 4, tiled(0, 16, 16, 1)};
+  return {64, 4, tiled(0, 8, 16, 1)};
 }
 
 int step_class(int precision, bool dots, bool real = false) {
@@ -272,44 +261,94 @@ const StepEntry *default_step(const tbtkkpm_matrix *m, int precision, bool dots,
                               bool real64) {
   const bool real = real_mode(m, precision);
   Shape s = shape_for(precision, B, real, dots, m->N);
-  if (real64 && real64_shape_for(B, m->N).bp()) s = real64_shape_for(B, m->N);
+  if (real64) s = real64_shape_for(B);
   return find_step(step_class(precision, dots, real), s.tpr, s.vpt, s.minb);
 }
 
-// A tile-staged entry runs with the matrix's plan for its tile height when
-// a ring of at least two stages fits its shared memory; one on real FP64
-// vectors also needs the batch to take them (real64).  Otherwise a forced
-// entry is refused (TBTKKPM_ERR_UNSUPPORTED, which the autotuner skips) and
-// a chosen one gives way: real FP64 vectors to the complex default, a
-// tile-staged step to the register-staged default of the batch.
+// The matrix's plan for a tile-staged entry, null where a ring of at least
+// two stages does not fit the entry's shared memory (or a tile does not fit
+// the builder).  Columns are staged one at a time, or four where that saves
+// copies: rows of up to 32 bytes, and patterns of short runs, of which a
+// producer warp issues one in about 50 ns (a honeycomb sublattice makes runs
+// of two rows; 32 real sources on 500^2 cells took 208 us per step with them,
+// 2.1 us a tile, where the bytes take 60).
+int fitting_plan(tbtkkpm_matrix *m, const StepEntry *fn, const TilePlan *&plan) {
+  plan = nullptr;
+  const bool r64 = fn->cls == kClassFP64Real;
+  const bool cplx = !(r64 || fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots);
+  const uint32_t esz = fn->cls == kClassFP64 ? sizeof(double2)
+                       : r64                 ? sizeof(double)
+                       : cplx                ? sizeof(float2)
+                                             : sizeof(float);
+  const uint32_t rowbytes = (uint32_t)(fn->tpr * fn->vpt) * esz;
+  const int rows = tiled_rows(fn->minb);
+  const bool pairs = tiled_pairs(fn->minb);
+  auto fits = [&](const TilePlan *p) {
+    return p && tiled_layout(*p, rowbytes, cplx ? sizeof(double2) : sizeof(double),
+                             tiled_budget(tiled_bps(fn->minb))).stages != 0;
+  };
+  const TilePlan *one = nullptr, *four = nullptr;
+  int rc = TBTKKPM_OK;
+  const bool narrow = rowbytes <= 32 && !pairs;
+  if (!narrow && (rc = tile_plan(m, rows, cplx, &one, pairs, 1))) return rc;
+  if (narrow || (!pairs && one && one->nruns > (uint64_t)one->ntiles * (4 + rows / 16))) {
+    if ((rc = tile_plan(m, rows, cplx, &four, false, 4))) return rc;
+    if (fits(four) && (!one || 2 * (uint64_t)four->nruns <= one->nruns)) {
+      plan = four;
+      return TBTKKPM_OK;
+    }
+  }
+  if (narrow && tiled_unit(rowbytes) == 1 && (rc = tile_plan(m, rows, cplx, &one, false, 1))) return rc;
+  if (fits(one)) plan = one;
+  return TBTKKPM_OK;
+}
+
+// A tile-staged entry runs with a plan that fits (fitting_plan); one on real
+// FP64 vectors also needs the batch to take them (real64).  Otherwise a
+// forced entry is refused (TBTKKPM_ERR_UNSUPPORTED, which the autotuner
+// skips) and a chosen one gives way: to the tile-staged entry of its class
+// and width that fits with the most consumer warps per SM (wide rows: on the
+// 512^2 Rashba lattice one FP64 source takes 16 us per step with 6 blocks per
+// SM, where 8 do not fit, against 30 register-staged), then real FP64 vectors
+// to the complex default, then to the register-staged default of the batch.
 int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool forced, bool real64,
                   const StepEntry *&fn, const TilePlan *&plan) {
   plan = nullptr;
+  const bool real = real_mode(m, precision);
+  const int cls = step_class(precision, dots, real);
+  int rc;
   while (fn && is_tiled_variant(fn->minb)) {
     const bool r64 = fn->cls == kClassFP64Real;
-    const bool cplx = !(r64 || fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots);
-    const uint32_t esz = fn->cls == kClassFP64 ? sizeof(double2)
-                         : r64                 ? sizeof(double)
-                         : cplx                ? sizeof(float2)
-                                               : sizeof(float);
-    const uint32_t vsz = cplx ? sizeof(double2) : sizeof(double);
-    const uint32_t rowbytes = (uint32_t)(fn->tpr * fn->vpt) * esz;
-    const TilePlan *p = nullptr;
     if (!r64 || real64) {
-      int rc = tile_plan(m, tiled_rows(fn->minb), cplx, &p, tiled_pairs(fn->minb), rowbytes < 16 ? 2 : 1);
-      if (rc) return rc;
-    }
-    if (p && tiled_layout(*p, rowbytes, vsz, tiled_budget(tiled_bps(fn->minb))).stages) {
-      plan = p;
-      return TBTKKPM_OK;
+      if ((rc = fitting_plan(m, fn, plan))) return rc;
+      if (plan) return TBTKKPM_OK;
     }
     if (forced)
       return fail(TBTKKPM_ERR_UNSUPPORTED,
                   "recursion: the tile-staged step %d x %d / %d does not fit this matrix", fn->tpr,
                   fn->vpt, fn->minb);
-    const Shape s = r64 ? shape_for(precision, B, false, dots, m->N)
-                        : register_shape_for(precision, B, !cplx, dots);
-    fn = find_step(step_class(precision, dots, !cplx && !r64), s.tpr, s.vpt, s.minb);
+    if (!r64 || real64) {
+      const StepEntry *t;
+      int n;
+      step_table(cls, &t, &n);
+      std::vector<const StepEntry *> others;
+      for (int i = 0; i < n; i++)
+        if (&t[i] != fn && t[i].cls == fn->cls && t[i].tpr * t[i].vpt == fn->tpr * fn->vpt &&
+            is_tiled_variant(t[i].minb) && !tiled_pairs(t[i].minb))
+          others.push_back(&t[i]);
+      auto warps = [](const StepEntry *e) { return tiled_bps(e->minb) * tiled_warps(e->minb); };
+      std::stable_sort(others.begin(), others.end(),
+                       [&](const StepEntry *a, const StepEntry *b) { return warps(a) > warps(b); });
+      for (const StepEntry *e : others) {
+        if ((rc = fitting_plan(m, e, plan))) return rc;
+        if (plan) {
+          fn = e;
+          return TBTKKPM_OK;
+        }
+      }
+    }
+    const Shape s = r64 ? shape_for(precision, B, false, dots, m->N) : register_shape_for(precision, B, real, dots);
+    fn = find_step(cls, s.tpr, s.vpt, s.minb);
   }
   return TBTKKPM_OK;
 }
@@ -365,8 +404,8 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
   if (Bp < B) return fail(TBTKKPM_ERR_ARGUMENT, "configuration of %u columns for %u sources", Bp, B);
   const bool real = kind == kVecF32;
   const size_t esize = vec_elem_size(kind);
-  // rows of 8 bytes are staged two at a time: one padding row for an odd N
-  const size_t vbytes = (size_t)m->N * Bp * esize + (Bp * esize < 16 ? 16 : 0);
+  // rows may be staged four at a time, past the last row
+  const size_t vbytes = ((size_t)m->N + 3) * Bp * esize + 16;
   const size_t words = ((size_t)m->N + 31) / 32;
   const uint32_t T = (uint32_t)tl.row.size();
   const uint32_t steps = doubling ? M / 2 : (M >= 2 ? M - 1 : 0);  // last j index computed
@@ -377,8 +416,13 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
   const uint32_t per_launch =
       doubling ? (uint32_t)std::max<size_t>(32, std::min<size_t>(steps, ((size_t)64 << 20) / std::max<size_t>(step_part, 1)))
                : 4096;
-  const size_t dots_bytes =
-      res.ok ? step_part * std::min(per_launch, std::max(steps, 1u)) : sizeof(double2) * 2 * (size_t)Bp * max_grid;
+  // launched steps keep the block sums of several steps (up to 32 MB of them)
+  // for one reduction
+  const size_t dots_stride = 2 * (size_t)Bp * max_grid;
+  const uint32_t dots_steps = (uint32_t)std::min<size_t>(
+      64, std::max<size_t>(1, ((size_t)32 << 20) / (sizeof(double2) * dots_stride)));
+  const size_t dots_bytes = res.ok ? step_part * std::min(per_launch, std::max(steps, 1u))
+                                   : sizeof(double2) * dots_stride * std::min(dots_steps, std::max(steps, 1u));
   if ((rc = ws.vec[0].reserve(vbytes)) || (rc = ws.vec[1].reserve(vbytes)) ||
       (rc = ws.bitmap.reserve(4 * words)) || (rc = ws.tgt.reserve(12 * std::max(T, 1u))) ||
       (rc = ws.from.reserve(4 * std::max(B, 1u))) || (rc = ws.err.reserve(16)) ||
@@ -525,28 +569,39 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
     launch_resident_dots(st, res, n, r.n1 - n + 1, B, ws.dots.as<double>(), ws.col_out.as<uint32_t>(),
                          ws.mu.as<double2>(), M, M);
   }
-  if (!res.ok) count_launches((uint64_t)(steps - q) * (doubling ? 2 : 1));
+  if (!res.ok) count_launches(steps - q);
+  uint32_t n_dots = q + 1;      // first step whose block sums are not reduced yet
+  unsigned dots_grid = 0;       // their blocks
+  auto reduce_dots = [&](uint32_t end) {  // the steps [n_dots, end)
+    if (end > n_dots) {
+      kpm_dots_finalize<<<dim3(Bp, end - n_dots), kFinalizeBlock, 0, st>>>(
+          Bp, dots_grid, ws.dots.as<double2>(), dots_stride, ws.col_out.as<uint32_t>(),
+          ws.mu.as<double2>(), M, M, n_dots);
+      count_launches(1);
+    }
+    n_dots = end;
+  };
   for (uint32_t n = q + 1; !res.ok && n <= steps; n++) {
     a.x = cur;
     a.y = prev;
     a.n_out = n;
+    if (doubling) a.dots = ws.dots.as<double2>() + (size_t)(n - n_dots) * dots_stride;
     unsigned grid = 0;
     (n == 1 ? fn->first : fn->rest)(st, m->device, max_grid, a, &grid);
     if (grid == 0) return fail(TBTKKPM_ERR_UNSUPPORTED, "recursion: step %d x %d / %d not launched",
                                fn->tpr, fn->vpt, fn->minb);
     std::swap(cur, prev);
-    if (doubling) {
-      if (n == 1) {
-        // mu_0 and mu_1 of the direct gather seed the doubling identities
-        e = cudaMemcpy2DAsync(ws.mu.ptr, sizeof(double2) * M, ws.mu_direct.ptr,
-                              sizeof(double2) * ld_direct, sizeof(double2) * std::min(M, 2u),
-                              K, cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) return cuda_fail(e, "recursion: seed moments");
-      }
-      kpm_dots_finalize<<<Bp, kFinalizeBlock, 0, st>>>(Bp, grid, ws.dots.as<double2>(),
-                                                              ws.col_out.as<uint32_t>(),
-                                                              ws.mu.as<double2>(), M, M, n);
+    if (!doubling) continue;
+    dots_grid = grid;
+    if (n == 1) {
+      // mu_0 and mu_1 of the direct gather seed the doubling identities
+      e = cudaMemcpy2DAsync(ws.mu.ptr, sizeof(double2) * M, ws.mu_direct.ptr,
+                            sizeof(double2) * ld_direct, sizeof(double2) * std::min(M, 2u),
+                            K, cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return cuda_fail(e, "recursion: seed moments");
     }
+    // the first step's kernel may run another grid than the rest
+    if (n == 1 || n == steps || n + 1 - n_dots == dots_steps) reduce_dots(n + 1);
   }
   if (doubling && steps == 0) {
     e = cudaMemcpy2DAsync(ws.mu.ptr, sizeof(double2) * M, ws.mu_direct.ptr,

@@ -46,14 +46,21 @@ int fill_tiles(cudaStream_t st, const tbtkkpm_matrix *m, uint32_t ntiles, unsign
   return TBTKKPM_OK;
 }
 
+// the built (rows per tile, unit) pairs
+#define TBTKKPM_PLANS(X)                                                                 \
+  X(8, 1) X(16, 1) X(32, 1) X(64, 1) X(128, 1) X(256, 1) X(8, 4) X(16, 4) X(32, 4)      \
+  X(64, 4) X(128, 4) X(256, 4)
+
 // pairs: the row-pair plan of complex values (R >= 16; k_plan_pair_width);
-// unit: columns staged together (2: real values in tiles of 64 rows and up).
-// Tiles of 128 and 256 rows: real values only.
+// unit: columns staged together
 int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, TilePlanStore &p) {
-  if (unit != 1 && (unit != 2 || cplx || pairs || R < 64))
-    return fail(TBTKKPM_ERR_UNSUPPORTED, "tile plan: no builder for units of %u columns", unit);
-  if (pairs && (!cplx || R < 16))
-    return fail(TBTKKPM_ERR_UNSUPPORTED, "tile plan: row pairs need complex values and R >= 16");
+  bool known = false;
+#define TBTKKPM_KNOWN(RR, U) known |= R == RR && unit == U;
+  TBTKKPM_PLANS(TBTKKPM_KNOWN)
+#undef TBTKKPM_KNOWN
+  if (!known)
+    return fail(TBTKKPM_ERR_UNSUPPORTED, "tile plan: no builder for %d rows per tile in units of %u columns",
+                R, unit);
   cudaStream_t st = m->stream;
   const uint32_t ntiles = (m->N + R - 1) / R;
   const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)sm_count(m->device) * 8);
@@ -68,16 +75,10 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, T
       (e = cudaMemsetAsync(tw.as<uint32_t>() + ntiles, 0, 4, st)) ||
       (e = cudaMemsetAsync(truns.as<uint32_t>() + ntiles, 0, 4, st)))
     return cuda_fail(e, "tile plan: staging");
-  if (unit == 2 && R == 64) rc = count_tiles<64, 2>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (unit == 2 && R == 128) rc = count_tiles<128, 2>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (unit == 2 && R == 256) rc = count_tiles<256, 2>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (R == 128 && !cplx) rc = count_tiles<128>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (R == 256 && !cplx) rc = count_tiles<256>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (R == 8) rc = count_tiles<8>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (R == 16) rc = count_tiles<16>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (R == 32) rc = count_tiles<32>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else if (R == 64) rc = count_tiles<64>(st, m, ntiles, grid, tw, truns, tuniq, flags);
-  else return fail(TBTKKPM_ERR_UNSUPPORTED, "tile plan: no builder for %d rows per tile", R);
+#define TBTKKPM_COUNT(RR, U) \
+  if (R == RR && unit == U) rc = count_tiles<RR, U>(st, m, ntiles, grid, tw, truns, tuniq, flags);
+  TBTKKPM_PLANS(TBTKKPM_COUNT)
+#undef TBTKKPM_COUNT
   count_launches(1);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "tile plan: count");
   if (pairs) {
@@ -117,25 +118,16 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, T
   if ((rc = p.hdr.reserve(16 * (size_t)ntiles)) || (rc = p.runs.reserve(8 * std::max(nruns, 1u))) ||
       (rc = p.eslot.reserve(2 * slots)) || (rc = p.eval.reserve(vsz * slots)))
     return rc;
-#define TBTKKPM_FILL(RR)                                                                      \
-  (cplx ? fill_tiles<RR, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p)            \
-        : fill_tiles<RR, false>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p))
   if (pairs) {
     if (R == 16) rc = fill_tiles<16, true, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
     else if (R == 32) rc = fill_tiles<32, true, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
     else rc = fill_tiles<64, true, true>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
-  } else if (unit == 2) {
-    if (R == 64) rc = fill_tiles<64, false, false, 2>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
-    else if (R == 128) rc = fill_tiles<128, false, false, 2>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
-    else rc = fill_tiles<256, false, false, 2>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
-  } else if (R == 128) {
-    rc = fill_tiles<128, false>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
-  } else if (R == 256) {
-    rc = fill_tiles<256, false>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
-  } else if (R == 8) rc = TBTKKPM_FILL(8);
-  else if (R == 16) rc = TBTKKPM_FILL(16);
-  else if (R == 32) rc = TBTKKPM_FILL(32);
-  else rc = TBTKKPM_FILL(64);
+  }
+#define TBTKKPM_FILL(RR, U)                                                                              \
+  if (R == RR && unit == U && !pairs)                                                                    \
+    rc = cplx ? fill_tiles<RR, true, false, U>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p)       \
+              : fill_tiles<RR, false, false, U>(st, m, ntiles, grid, ent, run, tw, truns, tuniq, p);
+  TBTKKPM_PLANS(TBTKKPM_FILL)
 #undef TBTKKPM_FILL
   if (rc) return rc;
   count_launches(1);
