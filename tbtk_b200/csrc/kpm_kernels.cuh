@@ -25,6 +25,7 @@
 
 #include <cstdint>
 #include <cuda_runtime.h>
+#include <type_traits>
 
 namespace tbtkkpm {
 
@@ -709,48 +710,105 @@ static __global__ void kpm_table_gen(uint32_t M, uint32_t E, const double *energ
 // (n outer, e inner, ChebyshevExpander.cpp:324-361), each operation rounded
 // once.  KT coefficient vectors per thread share each table load; a block
 // stages a chunk of their coefficients in shared memory.
-constexpr int kEnergyBlock = 128;
+//
+// The order fixes a chain of M sums per (k, e), so a thread keeps the table
+// values of the next 16 or 32 terms in registers: with a load per term in the
+// chain's way a term took 316 cycles (K = 64, M = 4096, E = 2048, LDOS: 0.66
+// ms).  What bounds it then is shared memory, whose broadcast of a coefficient
+// costs a warp as much as the two FP64 operations it feeds, and for few
+// vectors the latency of the table's loads; energy_shape in recursion.cu picks
+// KT and the block.  (A cp.async ring in place of the registers, and
+// coefficients read two terms at a time, measured 10-60% slower.)
+constexpr int kEnergyBlock = 128;  // most threads of a block
 constexpr int kEnergyChunk = 128;
+// terms ahead: more where a term's work covers less of a load's latency; a
+// divisor of kEnergyChunk
+template <int KT> __host__ __device__ constexpr int energy_ahead() { return KT <= 2 ? 32 : 16; }
+
+// Type 4 is the LDOS: 0 + Im(G_NP[k][e])/pi (PropertyExtractor
+// ChebyshevExpander.cpp:682-683), of which only the imaginary part
+// Im(G) -= (c.re*1 + c.im*0) * Im(T) is accumulated.
+template <int TYPE> struct EnergyTerm {
+  static constexpr bool LDOS = TYPE == 4;
+  using C = typename std::conditional<LDOS, double, double2>::type;  // coefficient, sum
+  // the part of a table value the type needs
+  using T = typename std::conditional<TYPE <= 1, double2, double>::type;
+  __device__ __forceinline__ static T load(const double2 *t) {
+    if constexpr (TYPE <= 1) return __ldg(t);
+    else if constexpr (TYPE == 2) return __ldg(&t->x);
+    else return __ldg(&t->y);
+  }
+  __device__ __forceinline__ static C coefficient(double2 c) {
+    if constexpr (LDOS) return __dadd_rn(__dmul_rn(c.x, 1.0), __dmul_rn(c.y, 0.0));
+    // c*i = (c.re*0 - c.im*1, c.re*1 + c.im*0)
+    else if constexpr (TYPE == 3) return cmul_exact(c, make_double2(0.0, 1.0));
+    else return c;
+  }
+  __device__ __forceinline__ static C add(C acc, C c, T t) {
+    if constexpr (TYPE == 1) {          // Retarded: G += T*c
+      return cadd_exact(acc, cmul_exact(t, c));
+    } else if constexpr (TYPE == 0) {   // Advanced: G += c*conj(T)
+      return cadd_exact(acc, cmul_exact(c, make_double2(t.x, -t.y)));
+    } else if constexpr (TYPE == 2) {   // Principal: G += -c*Re(T)
+      return cadd_exact(acc, make_double2(__dmul_rn(-c.x, t), __dmul_rn(-c.y, t)));
+    } else if constexpr (TYPE == 3) {   // NonPrincipal: G -= (c*i)*Im(T)
+      return make_double2(__dsub_rn(acc.x, __dmul_rn(c.x, t)), __dsub_rn(acc.y, __dmul_rn(c.y, t)));
+    } else {
+      return __dsub_rn(acc, __dmul_rn(c, t));
+    }
+  }
+  __device__ __forceinline__ static C result(C acc) {
+    if constexpr (LDOS) return __dadd_rn(0.0, __ddiv_rn(acc, 3.14159265358979323846));
+    else return acc;
+  }
+};
 
 template <int TYPE, int KT>
 __global__ void __launch_bounds__(kEnergyBlock)
-kpm_greens(uint32_t M, uint32_t E, uint32_t K, const double2 *__restrict__ table,
-           const double2 *__restrict__ mu, double2 *__restrict__ G) {
-  __shared__ double2 cs[KT][kEnergyChunk];
-  const uint32_t e = blockIdx.x * kEnergyBlock + threadIdx.x;
+kpm_energy(uint32_t M, uint32_t E, uint32_t K, const double2 *__restrict__ table,
+           const double2 *__restrict__ mu, typename EnergyTerm<TYPE>::C *__restrict__ out) {
+  using X = EnergyTerm<TYPE>;
+  using C = typename X::C;
+  using T = typename X::T;
+  constexpr int U = energy_ahead<KT>();
+  __shared__ C cs[KT][kEnergyChunk];
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
   const uint32_t k0 = blockIdx.y * KT;
-  double2 acc[KT];
+  C acc[KT];
 #pragma unroll
-  for (int j = 0; j < KT; j++) acc[j] = make_double2(0.0, 0.0);
+  for (int j = 0; j < KT; j++) acc[j] = C{};
+  const double2 *col = table + min(e, E - 1);
+  T next[U];  // the table values of the next U terms (past M: the last one's, not used)
+#pragma unroll
+  for (int u = 0; u < U; u++) next[u] = X::load(col + (uint64_t)min((uint32_t)u, M - 1) * E);
   for (uint32_t n0 = 0; n0 < M; n0 += kEnergyChunk) {
     const uint32_t nc = min((uint32_t)kEnergyChunk, M - n0);
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < KT * kEnergyChunk; i += kEnergyBlock) {
+    for (uint32_t i = threadIdx.x; i < KT * kEnergyChunk; i += blockDim.x) {
       const uint32_t j = i / kEnergyChunk, n = i % kEnergyChunk;
-      double2 c = make_double2(0.0, 0.0);
-      if (k0 + j < K && n < nc) c = mu[(uint64_t)(k0 + j) * M + n0 + n];
-      if constexpr (TYPE == 3) {
-        // c*i = (c.re*0 - c.im*1, c.re*1 + c.im*0)
-        c = cmul_exact(c, make_double2(0.0, 1.0));
-      }
+      C c{};
+      if (k0 + j < K && n < nc) c = X::coefficient(mu[(uint64_t)(k0 + j) * M + n0 + n]);
       cs[j][n] = c;
     }
     __syncthreads();
-    if (e < E) {
-      for (uint32_t n = 0; n < nc; n++) {
-        const double2 t = __ldg(table + (uint64_t)(n0 + n) * E + e);
+    for (uint32_t n = 0; n < nc; n += U) {
+      if (n0 + n + 2 * U <= M) {
+        const double2 *ahead = col + (uint64_t)(n0 + n + U) * E;
 #pragma unroll
-        for (int j = 0; j < KT; j++) {
-          const double2 c = cs[j][n];
-          if constexpr (TYPE == 1) {          // Retarded: G += T*c
-            acc[j] = cadd_exact(acc[j], cmul_exact(t, c));
-          } else if constexpr (TYPE == 0) {   // Advanced: G += c*conj(T)
-            acc[j] = cadd_exact(acc[j], cmul_exact(c, make_double2(t.x, -t.y)));
-          } else if constexpr (TYPE == 2) {   // Principal: G += -c*Re(T)
-            acc[j] = cadd_exact(acc[j], make_double2(__dmul_rn(-c.x, t.x), __dmul_rn(-c.y, t.x)));
-          } else {                            // NonPrincipal: G -= (c*i)*Im(T)
-            acc[j] = make_double2(__dsub_rn(acc[j].x, __dmul_rn(c.x, t.y)),
-                                  __dsub_rn(acc[j].y, __dmul_rn(c.y, t.y)));
+        for (int u = 0; u < U; u++) {
+          const T t = next[u];
+          next[u] = X::load(ahead + (uint64_t)u * E);
+#pragma unroll
+          for (int j = 0; j < KT; j++) acc[j] = X::add(acc[j], cs[j][n + u], t);
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          const T t = next[u];
+          next[u] = X::load(col + (uint64_t)min(n0 + n + U + u, M - 1) * E);
+          if (n + u < nc) {
+#pragma unroll
+            for (int j = 0; j < KT; j++) acc[j] = X::add(acc[j], cs[j][n + u], t);
           }
         }
       }
@@ -759,54 +817,12 @@ kpm_greens(uint32_t M, uint32_t E, uint32_t K, const double2 *__restrict__ table
   if (e < E) {
 #pragma unroll
     for (int j = 0; j < KT; j++)
-      if (k0 + j < K) G[(uint64_t)(k0 + j) * E + e] = acc[j];
-  }
-}
-
-// LDOS[k][e] = 0 + Im(G_NP[k][e])/pi (PropertyExtractor ChebyshevExpander.cpp:682-683).
-// Only the imaginary part of G_NonPrincipal is accumulated:
-// Im(G) -= (c.re*1 + c.im*0) * Im(T).
-template <int KT>
-__global__ void __launch_bounds__(kEnergyBlock)
-kpm_ldos(uint32_t M, uint32_t E, uint32_t K, const double2 *__restrict__ table,
-         const double2 *__restrict__ mu, double *__restrict__ out) {
-  __shared__ double cs[KT][kEnergyChunk];
-  const uint32_t e = blockIdx.x * kEnergyBlock + threadIdx.x;
-  const uint32_t k0 = blockIdx.y * KT;
-  double acc[KT];
-#pragma unroll
-  for (int j = 0; j < KT; j++) acc[j] = 0.0;
-  for (uint32_t n0 = 0; n0 < M; n0 += kEnergyChunk) {
-    const uint32_t nc = min((uint32_t)kEnergyChunk, M - n0);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < KT * kEnergyChunk; i += kEnergyBlock) {
-      const uint32_t j = i / kEnergyChunk, n = i % kEnergyChunk;
-      double c = 0.0;
-      if (k0 + j < K && n < nc) {
-        const double2 m = mu[(uint64_t)(k0 + j) * M + n0 + n];
-        c = __dadd_rn(__dmul_rn(m.x, 1.0), __dmul_rn(m.y, 0.0));
-      }
-      cs[j][n] = c;
-    }
-    __syncthreads();
-    if (e < E) {
-      for (uint32_t n = 0; n < nc; n++) {
-        const double ti = __ldg(&table[(uint64_t)(n0 + n) * E + e].y);
-#pragma unroll
-        for (int j = 0; j < KT; j++) acc[j] = __dsub_rn(acc[j], __dmul_rn(cs[j][n], ti));
-      }
-    }
-  }
-  if (e < E) {
-#pragma unroll
-    for (int j = 0; j < KT; j++)
-      if (k0 + j < K)
-        out[(uint64_t)(k0 + j) * E + e] = __dadd_rn(0.0, __ddiv_rn(acc[j], 3.14159265358979323846));
+      if (k0 + j < K) out[(uint64_t)(k0 + j) * E + e] = X::result(acc[j]);
   }
 }
 
 // ---------------------------------------------------------------- table-free energy sums
-// The sums of kpm_greens / kpm_ldos without the M x E table (an
+// The sums of kpm_energy without the M x E table (an
 // energy-sum variant for memory-light serving).  With x = E_e/s,
 // theta = acos x, q = sin theta = sqrt(1 - x^2) and the table entries
 // T[n][e] = (1/s)(-2i/q) e^{-i n theta}/(1 + delta_n0), every type is a

@@ -1057,6 +1057,38 @@ extern "C" int tbtkkpm_table_destroy(tbtkkpm_table *t) {
 
 namespace tbtkkpm {
 
+// How an energy sum is split: KT vectors per thread and `block` energies per
+// block.  More vectors per thread share a table value and its load, fewer
+// spread the sums over more warps; a warp per scheduler is worth about two
+// more vectors.  us of the LDOS kernel with KT = 1 / 2 / 4 / 8, M = 1000, E =
+// 1000: 28 / 35 / 51 / 76 for K = 8, 37 / 38 / 53 / 79 for K = 30, 75 / 46 /
+// 55 / 82 for K = 64; M = 4096, E = 2000: 451 / 234 / 275 / 394 for K = 64,
+// 802 / 478 / 332 / 398 for K = 128 (one load per term and KT = 8: 88, 91, 96,
+// 656 and 665).
+struct EnergyShape {
+  int kt;
+  unsigned block;
+};
+
+static EnergyShape energy_shape(uint32_t E, uint32_t K, int sms) {
+  const uint64_t ew = (E + 31) / 32, few = (uint64_t)sms * 7;  // 1036 warps on 148 SMs
+  if (ew * K <= few) return {1, 64};
+  if (ew * ((K + 1) / 2) <= few) return {2, 64};
+  if (ew * ((K + 3) / 4) <= 2 * few) return {4, 128};
+  return {8, 128};
+}
+
+template <int TYPE>
+static void launch_energy(cudaStream_t st, EnergyShape sh, uint32_t M, uint32_t E, uint32_t K,
+                          const double2 *table, const double2 *mu, void *out) {
+  auto *o = static_cast<typename EnergyTerm<TYPE>::C *>(out);
+  const dim3 grid((E + sh.block - 1) / sh.block, (K + sh.kt - 1) / sh.kt);
+  if (sh.kt == 1) kpm_energy<TYPE, 1><<<grid, sh.block, 0, st>>>(M, E, K, table, mu, o);
+  else if (sh.kt == 2) kpm_energy<TYPE, 2><<<grid, sh.block, 0, st>>>(M, E, K, table, mu, o);
+  else if (sh.kt == 4) kpm_energy<TYPE, 4><<<grid, sh.block, 0, st>>>(M, E, K, table, mu, o);
+  else kpm_energy<TYPE, 8><<<grid, sh.block, 0, st>>>(M, E, K, table, mu, o);
+}
+
 // Launches the energy sum of `type` (0-3 Green's functions, 4 = LDOS) for K
 // coefficient vectors resident on the device ([K][M] with M = terms, or the
 // table's M when terms is 0; a table of more rows serves fewer terms).
@@ -1094,27 +1126,14 @@ int launch_energy_sum(cudaStream_t st, const tbtkkpm_table *t, const double2 *mu
     if (e != cudaSuccess) return cuda_fail(e, "energy sum: launch");
     return TBTKKPM_OK;
   }
-  const double2 *tb = t->table.as<double2>();
-#define TBTKKPM_G(TY, KK) \
-  kpm_greens<TY, KK><<<grid, kEnergyBlock, 0, st>>>(M, E, K, tb, mu, static_cast<double2 *>(out))
-#define TBTKKPM_TYPES(KK)                       \
-  switch (type) {                               \
-    case 0: TBTKKPM_G(0, KK); break;            \
-    case 1: TBTKKPM_G(1, KK); break;            \
-    case 2: TBTKKPM_G(2, KK); break;            \
-    case 3: TBTKKPM_G(3, KK); break;            \
-    default:                                    \
-      kpm_ldos<KK><<<grid, kEnergyBlock, 0, st>>>(M, E, K, tb, mu, static_cast<double *>(out)); \
+  const EnergyShape sh = energy_shape(E, K, sm_count(t->device));
+  switch (type) {
+    case 0: launch_energy<0>(st, sh, M, E, K, t->table.as<double2>(), mu, out); break;
+    case 1: launch_energy<1>(st, sh, M, E, K, t->table.as<double2>(), mu, out); break;
+    case 2: launch_energy<2>(st, sh, M, E, K, t->table.as<double2>(), mu, out); break;
+    case 3: launch_energy<3>(st, sh, M, E, K, t->table.as<double2>(), mu, out); break;
+    default: launch_energy<4>(st, sh, M, E, K, t->table.as<double2>(), mu, out);
   }
-  if (KT == 1) {
-    TBTKKPM_TYPES(1)
-  } else if (KT == 4) {
-    TBTKKPM_TYPES(4)
-  } else {
-    TBTKKPM_TYPES(8)
-  }
-#undef TBTKKPM_TYPES
-#undef TBTKKPM_G
   count_launches(1);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "energy sum: launch");
@@ -1122,20 +1141,30 @@ int launch_energy_sum(cudaStream_t st, const tbtkkpm_table *t, const double2 *mu
 }
 
 // Energy sum of host moments [K][terms] (terms 0: the table's M; a table of
-// more rows serves fewer terms with the same sums) into host `out`.
+// more rows serves fewer terms with the same sums) into host `out`.  Vectors
+// go up in parts of about 1 MB, so that a part's sums run while the next one
+// is copied (64 vectors of 4096 terms at 2000 energies: the sums take 0.3 ms,
+// the copies of pageable memory 0.6).
 int energy_sum_host(tbtkkpm_table *t, const double *mu, uint32_t K, int type, void *out,
                     size_t out_elem, uint32_t terms) {
   std::lock_guard<std::mutex> lk(t->lock);
   DeviceGuard g(t->device);
   const uint32_t M = terms ? terms : t->M;
-  const size_t mbytes = sizeof(double2) * (size_t)K * M;
-  const size_t obytes = out_elem * (size_t)K * t->E;
+  const size_t vbytes = sizeof(double2) * (size_t)M, rbytes = out_elem * (size_t)t->E;
   int rc;
-  if ((rc = t->mu.reserve(mbytes)) || (rc = t->out.reserve(obytes))) return rc;
-  cudaError_t e = cudaMemcpyAsync(t->mu.ptr, mu, mbytes, cudaMemcpyHostToDevice, t->stream);
-  if (e != cudaSuccess) return cuda_fail(e, "energy sum: upload");
-  if ((rc = launch_energy_sum(t->stream, t, t->mu.as<double2>(), K, type, t->out.ptr, M))) return rc;
-  e = cudaMemcpyAsync(out, t->out.ptr, obytes, cudaMemcpyDeviceToHost, t->stream);
+  if ((rc = t->mu.reserve(vbytes * K)) || (rc = t->out.reserve(rbytes * K))) return rc;
+  const uint32_t part = (uint32_t)std::max<size_t>(16, (((size_t)1 << 20) + vbytes - 1) / vbytes);
+  cudaError_t e;
+  for (uint32_t k = 0; k < K; k += part) {
+    const uint32_t n = std::min(part, K - k);
+    e = cudaMemcpyAsync(t->mu.as<char>() + k * vbytes, reinterpret_cast<const char *>(mu) + k * vbytes,
+                        n * vbytes, cudaMemcpyHostToDevice, t->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "energy sum: upload");
+    if ((rc = launch_energy_sum(t->stream, t, t->mu.as<double2>() + (size_t)k * M, n, type,
+                                t->out.as<char>() + k * rbytes, M)))
+      return rc;
+  }
+  e = cudaMemcpyAsync(out, t->out.ptr, rbytes * K, cudaMemcpyDeviceToHost, t->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(t->stream);
   if (e != cudaSuccess) return cuda_fail(e, "energy sum: download");
   return TBTKKPM_OK;
