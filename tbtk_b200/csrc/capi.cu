@@ -217,6 +217,8 @@ static int build_sell(tbtkkpm_matrix *m, cudaStream_t st) {
                                 (int64_t)ns + 1, st);
   uint32_t chunks = 0;
   e = cudaMemcpyAsync(&chunks, m->slice_ptr.as<uint32_t>() + ns, 4, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(&m->widest_slice, width.as<uint32_t>() + ns, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   width.release();
   tmp.release();

@@ -140,10 +140,10 @@ struct tbtkkpm_matrix {
   uint32_t batch_width[3] = {0, 0, 0};
   uint32_t nslices = 0;
   uint64_t chunks = 0;
+  uint32_t widest_slice = 0;  // entries of the longest row
   // on-chip recursion (resident.cu), filled on first use: slice_ptr on the
-  // host, its widest slice, groups at once per (kernel shape, shared memory)
+  // host, groups at once per (kernel shape, shared memory)
   std::vector<uint32_t> host_slice_ptr;
-  uint32_t widest_slice = 0;
   std::map<uint64_t, uint32_t> resident_groups;
   tbtkkpm::Workspace ws;
   tbtkkpm::PhaseTimer timer;

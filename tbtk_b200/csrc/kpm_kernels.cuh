@@ -627,7 +627,8 @@ __global__ void kpm_init_sources(uint32_t B, uint32_t Bp, const uint32_t *from, 
 }
 
 // ---------------------------------------------------------------- SELL build
-// Slice widths (longest row of each 32-row slice).
+// Slice widths (longest row of each 32-row slice), the widest at
+// width[nslices] (zero beforehand).
 static __global__ void k_sell_width(uint32_t N, uint32_t nslices, const uint32_t *rowptr,
                              uint32_t *width) {
   const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -635,6 +636,7 @@ static __global__ void k_sell_width(uint32_t N, uint32_t nslices, const uint32_t
   uint32_t w = 0;
   for (uint32_t r = s * 32; r < min(N, s * 32 + 32); r++) w = max(w, rowptr[r + 1] - rowptr[r]);
   width[s] = w;
+  atomicMax(width + nslices, w);
 }
 
 // Scatter of the CSR rows into the slices; padding slots get kPad / 0.

@@ -489,7 +489,7 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
       j.W = Bp;
       j.col = b;
       j.real = real ? 1u : 0u;
-      j.pad = 0;
+      j.width = m->widest_slice;
     }
     std::vector<PrefixResult> res;
     if ((rc = run_fp64_head(st, jobs, ws, res))) return rc;

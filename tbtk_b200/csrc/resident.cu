@@ -148,8 +148,6 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
                                     m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) return cuda_fail(e, "recursion: slice bounds");
-    m->widest_slice = 0;
-    for (uint32_t s = 0; s < m->nslices; s++) m->widest_slice = std::max(m->widest_slice, sp[s + 1] - sp[s]);
     m->host_slice_ptr = std::move(sp);
   }
   // a tenth below the launched step, for the error of both estimates

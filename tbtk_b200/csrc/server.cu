@@ -761,6 +761,7 @@ int run_joins(tbtkkpm_server *s, const std::vector<MultiJoin> &joins, const std:
     p.W = j.W;
     p.col = j.col;
     p.real = j.real;
+    p.width = m->mat->widest_slice;
     jobs.push_back(p);
     which.push_back(i);
   }
