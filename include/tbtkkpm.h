@@ -561,10 +561,10 @@ TBTKKPM_API int tbtkkpm_server_set_fp64_head(tbtkkpm_server *s, uint32_t steps);
  * max_moments x E table of 16-byte entries, same results up to rounding. */
 TBTKKPM_API int tbtkkpm_server_set_table_free(tbtkkpm_server *s, int enable);
 
-/* The steps of a tick replay a CUDA graph of one step of every lane class,
- * captured when the tick starts (enable = 1, the default; a device counter
- * gives each replay its step); enable = 0 launches every kernel of every
- * step directly.  A capture that fails turns graphs off for the server.
+/* enable = 1 (the default): a tick whose steps are shorter than their launches
+ * (many lane classes of small models) replays a CUDA graph of one step of
+ * every lane class, captured when the tick starts (a device counter gives each
+ * replay its step); enable = 0 launches every kernel of every step directly.  A capture that fails turns graphs off for the server.
  * Results do not depend on it.  (No reference counterpart.) */
 TBTKKPM_API int tbtkkpm_server_set_graphs(tbtkkpm_server *s, int enable);
 

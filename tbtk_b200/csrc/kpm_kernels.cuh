@@ -64,6 +64,23 @@ __device__ __forceinline__ double2 cmac(double2 acc, double2 v, double2 x) {
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Launches `kern`, with programmatic stream serialization if `dependent`.
+template <typename... P, typename... A>
+void launch_dependent(bool dependent, void (*kern)(P...), unsigned grid, unsigned block, size_t smem,
+                      cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = dependent ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---------------------------------------------------------------- vector packs
 // The VPT complex values a thread owns in one row of a batch, as raw loads:
 // complex128 as double2 each; complex64 as float2 (VPT = 1) or float4 pairs.

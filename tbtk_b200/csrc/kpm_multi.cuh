@@ -42,7 +42,7 @@ struct MultiModel {
   uint32_t tcount;
   const int32_t *base;       // [W] global step of the lane's local step 0, or kLaneIdle
   const uint32_t *lane_M;    // [W] moments the lane's request asks for
-  long long *dots;           // [2][W] fixed-point sums of the current step
+  long long *dots;           // [kDotsRing][2][W] fixed-point sums, step n at n % kDotsRing
   double2 *mu;               // [W][Mmax] doubled moments (0 and 1 seeded)
   double2 *mu_direct;        // [W][ld] directly gathered moments
   uint32_t tile0;            // first tile of this model in the launch
@@ -57,6 +57,13 @@ struct MultiModel {
   const void *p_val;
   uint32_t p_nruns, run0;
 };
+
+// Steps whose doubling sums a model holds until kpm_multi_finalize takes them
+// (a power of two).  One launch per step for them held up the next step.
+constexpr uint32_t kDotsRing = 8;
+__device__ __forceinline__ long long *multi_dots(const MultiModel *__restrict__ md, int32_t n, uint32_t W) {
+  return md->dots + ((uint32_t)n & (kDotsRing - 1)) * 2 * W;
+}
 
 // A model's target list pairs a row with an entry word: bits 0-7 the lane
 // (the column of the vectors), and with kPairEntry set the moment of the
@@ -297,7 +304,7 @@ kpm_multi_step(const MultiModel *__restrict__ models, const MultiHeader *__restr
       t_col = md->tcol;
       t_count = md->tcount;
       t_base = md->base;
-      t_dots = md->dots;
+      t_dots = multi_dots(md, n, W);
       first = 0;
 #pragma unroll
       for (int j = 0; j < VPT; j++)
@@ -433,26 +440,31 @@ kpm_multi_step(const MultiModel *__restrict__ models, const MultiHeader *__restr
 
 // After a step: the doubled moments of every active lane,
 // mu_{2m} = 2<j_m|j_m> - mu_0 and mu_{2m-1} = 2<j_m|j_{m-1}> - mu_1 for the
-// lane's local step m, and the fixed-point sums cleared for the next step.
-// One block per model, one thread per lane.
+// lane's local step m, and the fixed-point sums cleared, for the `steps` steps
+// up to step_offset (at most kDotsRing).  One block per model, one thread per
+// (step, lane).
 static __global__ void kpm_multi_finalize(const MultiModel *__restrict__ models,
                                    const MultiHeader *__restrict__ hdr, uint32_t step_offset,
-                                   uint32_t W, uint32_t Mmax, uint32_t ld) {
+                                   uint32_t steps, uint32_t W, uint32_t Mmax, uint32_t ld) {
   if (blockIdx.x >= hdr->nmodels) return;
   const MultiModel *md = models + blockIdx.x;
-  const int32_t n = multi_step_index(hdr, step_offset);
-  for (uint32_t c = threadIdx.x; c < W; c += blockDim.x) {
-    const long long a = md->dots[c], b = md->dots[W + c];
-    md->dots[c] = 0;
-    md->dots[W + c] = 0;
+  const int32_t last = multi_step_index(hdr, step_offset);
+  for (uint32_t t = threadIdx.x; t < W * steps; t += blockDim.x) {
+    const uint32_t c = t % W;
+    const int32_t n = last - (int32_t)(t / W);
+    long long *dots = multi_dots(md, n, W);
+    const long long a = dots[c], b = dots[W + c];
+    dots[c] = 0;
+    dots[W + c] = 0;
     const int32_t base = md->base[c];
     if (base == kLaneIdle) continue;
     const int32_t m = n - base;
     const uint32_t M = md->lane_M[c] & kLaneMBits;
     if (m < 1 || (uint32_t)m > M / 2) continue;
     double2 *row = md->mu + (uint64_t)c * Mmax;
-    if (m == 1) row[1] = md->mu_direct[(uint64_t)c * ld + 1];
-    const double2 mu0 = row[0], mu1 = row[1];
+    // mu_1 is the direct moment, which a head has copied or step 1 copies here
+    const double2 mu0 = row[0], mu1 = md->mu_direct[(uint64_t)c * ld + 1];
+    if (m == 1) row[1] = mu1;
     const double sa = (double)a * kFixUnit, sb = (double)b * kFixUnit;
     if (2 * (uint32_t)m < M) row[2 * m] = make_double2(2.0 * sa - mu0.x, -mu0.y);
     if (m >= 2 && 2 * (uint32_t)m - 1 < M) row[2 * m - 1] = make_double2(2.0 * sb - mu1.x, -mu1.y);
@@ -631,6 +643,7 @@ struct MultiLaunch {
   TiledLayout ly;
   int *err;
   uint32_t wait_limit;
+  bool dependent;  // start while the launch before it drains (tile-staged steps)
 };
 
 using MultiFn = void (*)(cudaStream_t, int device, const MultiModel *, const MultiHeader *,

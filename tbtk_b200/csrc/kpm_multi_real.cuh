@@ -101,7 +101,7 @@ kpm_multi_step_real(const MultiModel *__restrict__ models, const MultiHeader *__
       t_col = md->tcol;
       t_count = md->tcount;
       t_base = md->base;
-      t_dots = md->dots;
+      t_dots = multi_dots(md, n, W);
       first = 0;
 #pragma unroll
       for (int j = 0; j < VPT; j++)

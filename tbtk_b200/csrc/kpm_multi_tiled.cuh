@@ -119,6 +119,11 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
   const unsigned fullmask = 0xffffffffu;
   const uint32_t S = LY.stages;
   const uint32_t rowbytes = W * (uint32_t)sizeof(E);
+  // the next step's blocks may take this one's place as it drains (see
+  // kpm_step_tiled); vectors are read by bulk copies only
+  pdl_trigger();
+  pdl_wait();
+  if (warp == 0) asm volatile("fence.proxy.async.global;" ::: "memory");
   const uint32_t total = hdr->total_tiles, run = hdr->run;
   const uint4 *__restrict__ tdesc = hdr->tile_desc;
   const uint2 *__restrict__ truns = hdr->tile_runs;
@@ -176,7 +181,7 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
         m_slot = md->p_slot;
         m_x = reinterpret_cast<const E *>(md->vec[(n + 1) & 1]);
         m_y = reinterpret_cast<E *>(md->vec[n & 1]);
-        m_dots = md->dots;
+        m_dots = multi_dots(md, n, W);
         const int32_t *bs = md->base;
         const bool f0 = (uint32_t)lane < W && n - __ldg(bs + lane) == 1;
         const bool f1 = (uint32_t)lane + 32 < W && n - __ldg(bs + lane + 32) == 1;
@@ -447,9 +452,11 @@ void launch_multi_tiled(cudaStream_t st, int device, const MultiModel *models,
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tiled_budget(BPS));
     attr[d] = true;
   }
-  const uint32_t smem = kMultiHeader + ml.ly.stages * ml.ly.stage_bytes;
-  kern<<<(unsigned)(BPS * sm_count(device)), 32 * (CW + 1), smem, st>>>(
-      models, hdr, ml.ly, step_offset, W, ld, ml.err, ml.wait_limit);
+  // a dependent step takes its whole share of the SM, so that no more than
+  // BPS of its blocks gather on the SMs that end the step before first
+  const uint32_t smem = ml.dependent ? tiled_budget(BPS) : kMultiHeader + ml.ly.stages * ml.ly.stage_bytes;
+  launch_dependent(ml.dependent, kern, (unsigned)(BPS * sm_count(device)), 32 * (CW + 1), smem, st, models,
+                   hdr, ml.ly, step_offset, W, ld, ml.err, ml.wait_limit);
 }
 
 #define TBTKKPM_MULTI_TILED_ENTRY(CPLX, T, P, R, CW, BPS, CV)                          \

@@ -195,24 +195,6 @@ inline bool tiled_pairs(int v) { return (v - kTiledVariant) / 1000000 / 100 == 1
 inline int tiled_bps(int v) { return v % 10; }
 inline int tiled_warps(int v) { return (v - kTiledVariant) % 1000 / 10; }
 
-// Launches with programmatic stream serialization: the kernel's blocks may
-// start while the kernel before it drains (pdl_wait).
-template <typename... P, typename... A>
-void launch_dependent(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                      A... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-
 template <bool CPLX, int TPR, int VPT, int R, int CW, int BPS, bool FIRST, bool DOTS, int CV,
           bool F64 = false>
 void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs &a,
@@ -247,7 +229,7 @@ void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs
   static_assert(tiled_budget(BPS) >= kTiledHeader + 32u * CW * 16u, "reduction scratch");
   const uint32_t need = kTiledHeader + std::max(ly.stages * ly.stage_bytes, 32u * CW * 16u);
   const uint32_t smem = g == (uint64_t)BPS * sm_count(device) ? tiled_budget(BPS) : need;
-  launch_dependent(kern, (unsigned)g, 32 * (CW + 1), smem, st, p, ly, a.Bp,
+  launch_dependent(true, kern, (unsigned)g, 32 * (CW + 1), smem, st, p, ly, a.Bp,
                    static_cast<const E *>(a.x), static_cast<E *>(a.y), a.tg, a.n_out, a.dots, a.err,
                    a.wait_limit);
 }

@@ -148,7 +148,7 @@ struct RerunJob {
 // target bitmap and list (a row and an entry word for each of up to W
 // lane sites and W pair targets), pair moments.
 uint64_t lane_bytes(uint32_t N, uint32_t W, uint32_t Mmax, uint32_t ld, size_t esize) {
-  return 2ull * N * W * esize + 2ull * W * sizeof(long long) +
+  return 2ull * N * W * esize + 2ull * kDotsRing * W * sizeof(long long) +
          (uint64_t)W * Mmax * sizeof(double2) + (uint64_t)W * ld * sizeof(double2) +
          8ull * W + 4ull * ((N + 31) / 32) + 16ull * W + (uint64_t)W * Mmax * sizeof(double2);
 }
@@ -214,9 +214,10 @@ TiledLayout multi_layout(const MultiEntry *e, uint32_t W, bool real, uint32_t wm
                       tiled_budget(multi_tiled_bps(e->minb)) - (kMultiHeader - kTiledHeader));
 }
 
-// Default shape per width and class (measured choices of the single-model
-// kernels: few threads per row, several values each).
-std::array<int, 3> default_config(uint32_t W, bool real) {
+// Register-staged shape per width and class (few threads per row, several
+// values each): where rows are too narrow for bulk copies, or a model has no
+// plan or no ring that fits.
+std::array<int, 3> register_config(uint32_t W, bool real) {
   if (real) {
     switch (W) {
       case 1: return {1, 1, 2};
@@ -237,6 +238,32 @@ std::array<int, 3> default_config(uint32_t W, bool real) {
     case 32: return {8, 4, 2};
     default: return {8, 8, 2};
   }
+}
+
+// Default shape per width and class, before any tuning: the tile-staged steps.
+// A round of 24 models of up to 256^2 cells at 4-16 lanes spent 0.50 s in its
+// steps with the register-staged shapes above, 0.35 s with these (one change
+// at a time: real lanes 4, 8, 16 wide 0.498, 0.357, 0.371, 0.363; complex
+// 0.356, 0.351, 0.347).
+std::array<int, 3> default_config(uint32_t W, bool real) {
+  if (real) {
+    switch (W) {
+      case 4: return {1, 4, 164024};
+      case 8: return {1, 8, 164024};
+      case 16: return {2, 8, 164042};
+      case 32: return {8, 4, 164161};
+      case 64: return {8, 8, 164161};
+    }
+  } else {
+    switch (W) {
+      case 4: return {1, 4, 164024};
+      case 8: return {2, 4, 164042};
+      case 16: return {8, 2, 132082};
+      case 32: return {8, 4, 132082};
+      case 64: return {16, 4, 116082};
+    }
+  }
+  return register_config(W, real);
 }
 
 }  // namespace
@@ -334,7 +361,7 @@ int make_resident(tbtkkpm_server *s, Model *m) {
                            &m->base,   &m->laneM,  &m->bitmap, &m->tlist, &m->pmu};
   const size_t sizes[kViews] = {es * (size_t)N * W,
                                 es * (size_t)N * W,
-                                2 * sizeof(long long) * W,
+                                2 * kDotsRing * sizeof(long long) * W,
                                 sizeof(double2) * (size_t)W * s->Mmax,
                                 sizeof(double2) * (size_t)W * s->ld,
                                 4 * (size_t)W,
@@ -358,7 +385,7 @@ int make_resident(tbtkkpm_server *s, Model *m) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(m->vec[0].ptr, 0, es * (size_t)N * W, s->stream)) ||
       (e = cudaMemsetAsync(m->vec[1].ptr, 0, es * (size_t)N * W, s->stream)) ||
-      (e = cudaMemsetAsync(m->dots.ptr, 0, 2 * sizeof(long long) * W, s->stream))) {
+      (e = cudaMemsetAsync(m->dots.ptr, 0, 2 * kDotsRing * sizeof(long long) * W, s->stream))) {
     m->release_lanes();
     return cuda_fail(e, "server: lane memory");
   }
@@ -680,7 +707,7 @@ int plan_tick(tbtkkpm_server *s, std::vector<ClassPlan> &plans) {
       }
       if (ok) cp.ly = multi_layout(cp.entry, cp.W, cp.real, wmax, umax);
       if (!ok || cp.ly.stages == 0) {
-        const auto d = default_config(cp.W, cp.real);
+        const auto d = register_config(cp.W, cp.real);
         cp.entry = find_multi(d[0], d[1], d[2], cp.real);
         std::fill(tp.begin(), tp.end(), nullptr);
       }
@@ -778,6 +805,14 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
   cudaStream_t st = s->stream;
   int rc;
   cudaError_t e;
+  // A tick replays a captured graph where launching its steps would take the
+  // host longer (about 4.4 us per step and class) than the device takes to do
+  // them; elsewhere the graph's own launches, 12 us a step, and its capture,
+  // 0.4 ms a tick, are what is in the way (24 models: 0.50 s of steps replayed,
+  // 0.45 s launched).
+  double step_us = 8.0;
+  for (const ClassPlan &cp : plans) step_us += cp.bytes / 2.5e6;
+  const bool graph = s->use_graphs && nsteps > 1 && 4.4 * (double)plans.size() > step_us;
   // descriptors and headers of all plans in one upload
   size_t nm = 0;
   for (const ClassPlan &cp : plans) nm += cp.models.size();
@@ -805,7 +840,7 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
     }
     hdr.push_back({(uint32_t)cp.models.size(), cp.total_tiles, s->n_global,
                    s->d_tiles.as<uint32_t>() + tiles, s->d_tdesc.as<uint4>() + kDescWords * tiles,
-                   s->d_truns.as<uint2>() + runs, run, s->use_graphs ? s->d_step.as<int32_t>() : nullptr});
+                   s->d_truns.as<uint2>() + runs, run, graph ? s->d_step.as<int32_t>() : nullptr});
     tiles += cp.total_tiles;
     runs += cp.total_runs;
   }
@@ -837,6 +872,7 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
   // the launches of `steps` steps from step offset k0, forked from st and
   // joined back into it
   const int nstreams = (int)std::min<size_t>(plans.size(), tbtkkpm_server::kClassStreams);
+  uint64_t launches = 0;
   auto launch_steps = [&](uint32_t k0, uint32_t steps) -> cudaError_t {
     cudaError_t ee;
     if (nstreams > 1) {
@@ -844,7 +880,9 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
       for (int i = 0; i < nstreams; i++)
         if ((ee = cudaStreamWaitEvent(s->cls_stream[i], s->ev_fork, 0))) return ee;
     }
+    uint32_t done = k0;  // steps whose doubling sums are taken
     for (uint32_t k = k0; k < k0 + steps; k++) {
+      const bool take = k + 1 - done == kDotsRing || k + 1 == k0 + steps;
       size_t off = 0;
       for (size_t p = 0; p < plans.size(); p++) {
         const ClassPlan &cp = plans[p];
@@ -852,11 +890,16 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
         const MultiHeader *dh = s->d_hdr.as<MultiHeader>() + p;
         cudaStream_t cs = nstreams > 1 ? s->cls_stream[p % nstreams] : st;
         cp.entry->launch(cs, s->device, dm, dh, k, cp.W, s->ld,
-                         MultiLaunch{cp.ly, s->d_err.as<int>(), s->wait_limit});
-        kpm_multi_finalize<<<(unsigned)cp.models.size(), std::min<uint32_t>(std::max(cp.W, 32u), 64u),
-                             0, cs>>>(dm, dh, k, cp.W, s->Mmax, s->ld);
+                         MultiLaunch{cp.ly, s->d_err.as<int>(), s->wait_limit, !graph});
+        if (take) {
+          kpm_multi_finalize<<<(unsigned)cp.models.size(), std::min(512u, std::max(32u, cp.W * (k + 1 - done))), 0,
+                               cs>>>(dm, dh, k, k + 1 - done, cp.W, s->Mmax, s->ld);
+          launches++;
+        }
+        launches++;
         off += cp.models.size();
       }
+      if (take) done = k + 1;
     }
     if (nstreams > 1)
       for (int i = 0; i < nstreams; i++)
@@ -872,11 +915,11 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
     cudaGraphExecDestroy(s->tick_exec);
     s->tick_exec = nullptr;
   }
-  // the headers of this tick read d_step when graphs are on: it starts at 0
-  if (hdr[0].step && (e = cudaMemsetAsync(s->d_step.ptr, 0, sizeof(int32_t), st)))
+  // the headers of a replayed tick read d_step: it starts at 0
+  if (graph && (e = cudaMemsetAsync(s->d_step.ptr, 0, sizeof(int32_t), st)))
     return cuda_fail(e, "server: step counter");
   bool replay = false;
-  if (hdr[0].step && nsteps > 1) {
+  if (graph) {
     cudaGraph_t g = nullptr;
     if (cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed) == cudaSuccess) {
       cudaError_t ce = launch_steps(0, 1);
@@ -901,7 +944,7 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
     return cuda_fail(e, "server: step launch");
   }
   cudaEventRecord(s->ev[1], st);
-  count_launches((2ull * plans.size() + (replay ? 1 : 0)) * nsteps);
+  count_launches(replay ? (launches + 1) * nsteps : launches);
   if (replay) s->graph_ticks += 1;
   if ((e = cudaGetLastError())) return cuda_fail(e, "server: step launch");
   // the wait flag of the tile-staged steps, read after the tick
@@ -1761,7 +1804,7 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
   int rc;
   if ((rc = vec[0].reserve(es * (size_t)N * W)) ||
       (rc = vec[1].reserve(es * (size_t)N * W)) ||
-      (rc = dots.reserve(2 * sizeof(long long) * W)) || (rc = mu.reserve(sizeof(double2) * W * Mp)) ||
+      (rc = dots.reserve(2 * kDotsRing * sizeof(long long) * W)) || (rc = mu.reserve(sizeof(double2) * W * Mp)) ||
       (rc = mud.reserve(sizeof(double2) * W * ldp)) || (rc = base.reserve(4 * W)) ||
       (rc = laneM.reserve(4 * W)) || (rc = bitmap.reserve(4 * (size_t)((N + 31) / 32))) ||
       (rc = tlist.reserve(8 * W)) || (rc = dm.reserve(sizeof(MultiModel))) ||
@@ -1787,7 +1830,7 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
   DevBuf dj;
   if ((rc = dj.reserve(sizeof(MultiJoin) * W))) return rc;
   if ((e = cudaMemsetAsync(vec[1].ptr, 0, es * (size_t)N * W, st)) ||
-      (e = cudaMemsetAsync(dots.ptr, 0, 2 * sizeof(long long) * W, st)) ||
+      (e = cudaMemsetAsync(dots.ptr, 0, 2 * kDotsRing * sizeof(long long) * W, st)) ||
       (e = cudaMemcpyAsync(base.ptr, base_h.data(), 4 * W, cudaMemcpyHostToDevice, st)) ||
       (e = cudaMemcpyAsync(laneM.ptr, M_h.data(), 4 * W, cudaMemcpyHostToDevice, st)) ||
       (e = cudaMemcpyAsync(bitmap.ptr, bm.data(), 4 * bm.size(), cudaMemcpyHostToDevice, st)) ||
@@ -1872,14 +1915,16 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
       rc = cuda_fail(e, "server_autotune: tile map");
       break;
     }
-    const MultiLaunch ml{ly, s->d_err.as<int>(), kWaitLimit};
+    const MultiLaunch ml{ly, s->d_err.as<int>(), kWaitLimit, true};
     for (uint32_t k = 0; k < probe_steps; k++) {
       if (k == 1) cudaEventRecord(ev[0], st);
       en.launch(st, s->device, dm.as<MultiModel>(), dh.as<MultiHeader>(), k, W, ldp, ml);
-      kpm_multi_finalize<<<1, std::min<uint32_t>(std::max(W, 32u), 64u), 0, st>>>(
-          dm.as<MultiModel>(), dh.as<MultiHeader>(), k, W, Mp, ldp);
+      // the doubling sums are taken as in a tick's direct launches
+      if (k % kDotsRing == kDotsRing - 1 || k + 1 == probe_steps)
+        kpm_multi_finalize<<<1, std::min(512u, std::max(32u, W * kDotsRing)), 0, st>>>(
+            dm.as<MultiModel>(), dh.as<MultiHeader>(), k, k % kDotsRing + 1, W, Mp, ldp);
     }
-    count_launches(2ull * probe_steps);
+    count_launches(probe_steps + (probe_steps + kDotsRing - 1) / kDotsRing);
     cudaEventRecord(ev[1], st);
     if ((e = cudaEventSynchronize(ev[1])) != cudaSuccess) {
       rc = cuda_fail(e, "server_autotune: probe");

@@ -607,7 +607,8 @@ class Server:
                                                         int(minb)))
 
     def set_graphs(self, enable=True):
-        """Replay a captured CUDA graph per tick (default) or launch directly."""
+        """Let short ticks replay a captured CUDA graph (default) or launch
+        every step directly."""
         _check(load_library().tbtkkpm_server_set_graphs(self._h, int(bool(enable))))
 
     def set_adaptive_width(self, enable=True):
