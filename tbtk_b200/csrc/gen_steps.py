@@ -185,6 +185,7 @@ TILED_REAL = {
     (1, 8): _variants([(64, 2, 8), (64, 2, 6), (128, 4, 4)], [0, 51]),
     (2, 4): _variants([(64, 4, 6), (64, 4, 4)], [0, 51]),
     (2, 8): _variants([(64, 4, 4), (64, 4, 6)], [0, 51]),
+    (4, 8): _variants([(64, 8, 2), (64, 8, 3), (32, 4, 4)], [0, 51]),
 }
 # CV >= 100: the row-pair form (two adjacent rows per thread group, each
 # gathered row widened once for both; 16-row tiles and up).  On the 1024^2
@@ -213,6 +214,7 @@ TILED_CPLX = {
     (2, 2): _variants([(64, 4, 6)], [0, 60]) + _variants([(64, 4, 4)], [0]),
     (2, 4): _variants([(64, 4, 4), (64, 4, 6)], [0, 60]),
     (4, 2): _variants([(64, 8, 4)], [0, 60]),
+    (4, 4): _variants([(32, 4, 4), (64, 8, 2), (32, 4, 3)], [0]),
 }
 
 
@@ -226,9 +228,11 @@ TILED_FP64 = {
     (4, 1): [(64, 8, 4), (64, 8, 3), (64, 8, 2), (32, 4, 6)],
     (8, 1): [(64, 16, 2), (32, 8, 4), (64, 8, 3)],
     (16, 1): [(32, 8, 2), (64, 16, 1)],
+    (8, 2): [(32, 8, 2), (32, 8, 3)],
+    (4, 2): [(64, 8, 2), (64, 8, 3)],
     (32, 1): [(32, 8, 2), (16, 8, 2), (64, 16, 1)],
     (16, 2): [(32, 8, 2), (16, 8, 2)],
-    (32, 2): [(16, 16, 1), (16, 8, 1), (8, 8, 2), (8, 8, 1)],
+    (32, 2): [(16, 16, 1), (16, 8, 1), (8, 8, 2), (8, 8, 1), (8, 8, 3)],
     (16, 4): [(16, 8, 1), (8, 8, 2)],
     (32, 4): [(8, 8, 1), (8, 16, 1)],
     (16, 8): [(8, 8, 1)],

@@ -221,13 +221,14 @@ void launch_tiled(cudaStream_t st, int device, unsigned max_grid, const StepArgs
   if (max_grid) g = std::min<uint64_t>(g, max_grid);
   g = std::max<uint64_t>(g, 1);
   *grid = (unsigned)g;
-  // The ring holds the block's dot-product reduction at the end (2 doubles
-  // per consumer thread).  A full grid takes its whole share of the SM, so
+  // The ring holds the block's dot-product reduction at the end (two doubles
+  // per column and warp, or group of warps that share a row).  A full grid takes its whole share of the SM, so
   // that never more than BPS blocks fit one: blocks placed while the step
   // before drains would else pile up on the SMs that end first (10% slower
   // at 4 FP64 sources on the 1024^2 lattice).
-  static_assert(tiled_budget(BPS) >= kTiledHeader + 32u * CW * 16u, "reduction scratch");
-  const uint32_t need = kTiledHeader + std::max(ly.stages * ly.stage_bytes, 32u * CW * 16u);
+  constexpr uint32_t scratch = DOTS ? CW * 32 / (TPR > 32 ? TPR : 32) * TPR * VPT * 16 : 0;
+  static_assert(tiled_budget(BPS) >= kTiledHeader + scratch, "reduction scratch");
+  const uint32_t need = kTiledHeader + std::max(ly.stages * ly.stage_bytes, scratch);
   const uint32_t smem = g == (uint64_t)BPS * sm_count(device) ? tiled_budget(BPS) : need;
   launch_dependent(true, kern, (unsigned)g, 32 * (CW + 1), smem, st, p, ly, a.Bp,
                    static_cast<const E *>(a.x), static_cast<E *>(a.y), a.tg, a.n_out, a.dots, a.err,

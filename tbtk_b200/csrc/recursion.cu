@@ -132,42 +132,46 @@ Shape real64_shape_for(uint32_t B) {
   return {16, 8, tiled64r(8, 8, 2)};
 }
 
-// Default shape of a batch.  At mixed precision ms per step measured on the
-// 2048^2 lattice (real float vectors, doubling dots) for B = 32 / 64 / 128 /
-// 256: 1.05 / 1.43 / 3.01 / 5.71 against 1.82 / 2.90 / 4.79 / 11.8 for the
-// register-staged defaults, and on the 1024^2 Rashba lattice (complex64) for
-// B = 16 / 32 / 64 / 128 / 256: 0.38 / 0.55 / 1.09 / 2.14 / 4.27 against 1.06 /
-// 1.25 / 1.94 / 3.33 / 8.28.  Without the dots (directly gathered moments) the
-// real B = 64 step takes 1.29 ms (0.84 of the measured copy bandwidth).  A
-// matrix whose tiles do not fit a shape's ring takes the next one that does
-// (resolve_tiled).
-// N: the matrix's rows (0: large).
-Shape shape_for(int precision, uint32_t B, bool real = false, bool dots = false, uint32_t N = 0) {
+// Default shape of a batch; a matrix whose tiles do not fit its ring takes
+// the next one that does (resolve_tiled).  N: the matrix's rows (0: large),
+// widest: entries of its longest row.
+Shape shape_for(int precision, uint32_t B, bool real = false, bool dots = false, uint32_t N = 0,
+                uint32_t widest = 0) {
   if (!is_mixed(precision)) {
     // FP64 (complex128 vectors) on the 2048^2 lattice, ms per step for
-    // B = 1 / 2 / 4 / 8 / 16: 0.166 / 0.219 / 0.339 / 0.669 / 1.38
-    // tile-staged against 0.278 / 0.503 / 0.924 / 2.49 / 4.50
-    // register-staged, and for B = 32 / 64 / 128: 2.12 / 4.12 / 8.32
-    // (0.96-0.99 of the measured copy bandwidth) against 5.28 / 6.79 / 18.9.
-    // Dependent launches make tile staging the faster at every size: 181^2
-    // sites, B = 1 / 2 / 4: 2.9 / 3.4 / 4.6 us against 4.6 / 8.2 / 10.3.
+    // B = 1 / 2 / 4: 0.166 / 0.219 / 0.339 tile-staged against 0.278 / 0.503 /
+    // 0.924 register-staged.  Dependent launches make tile staging the faster
+    // at every size: 181^2 sites, B = 1 / 2 / 4: 2.9 / 3.4 / 4.6 us against 4.6
+    // / 8.2 / 10.3.  Two values per thread from 8 sources on: on the 301x203
+    // Rashba lattice 13.5 / 22 / 38 / 73 us for B = 8 / 16 / 32 / 64 against
+    // 14.1 / 31 / 44 / 86 for (8, 1), (16, 1), (16, 2) in 16-row tiles, (16, 4).
+    // At 16 sources three blocks per SM where rows are short enough for a
+    // ring of three stages (512^2 square: 67 us against 72 with two blocks;
+    // Rashba, two stages: 110 against 91).
     if (B <= 1) return {1, 1, tiled(0, 64, 2, 8)};
     if (B == 2) return {2, 1, tiled(0, 64, 4, 6)};
     if (B <= 4) return {4, 1, tiled(0, 64, 8, 4)};
-    if (B <= 8) return {8, 1, tiled(0, 64, 16, 2)};
-    if (B <= 16) return {16, 1, tiled(0, 32, 8, 2)};
-    if (B <= 32) return {16, 2, tiled(0, 16, 8, 2)};
-    if (B <= 64) return {16, 4, tiled(0, 8, 8, 2)};
+    if (B <= 8) return {4, 2, tiled(0, 64, 8, 2)};
+    if (B <= 16) return {8, 2, tiled(0, 32, 8, widest <= 6 ? 3 : 2)};
+    if (B <= 32) return {16, 2, tiled(0, 32, 8, 2)};
+    if (B <= 64) return {32, 2, tiled(0, 8, 8, 3)};
     return {32, 4, tiled(0, 8, 16, 1)};
   }
-  // Small batches: rows of 4-64 bytes, small tile-staged blocks, several per
-  // SM.  Doubling LDOS, us per step: real B = 1 / 2 / 4 / 8 on 1024^2 sites
-  // 24 / 29 / 37 / 59 against 60 / 64 / 95 / 150 register-staged, on 181^2
-  // 4.0 / 5.4 / 5.7 / 6.3 against 6.3 / 8.4 / 10 / 16; complex B = 1 / 2 / 4 /
-  // 8 on the 512^2 Rashba lattice 14 / 20 / 25 / 40 against 31 / 39 / 46 /
-  // 100.  Below 2^18 rows four and eight real sources are faster in 64-row
-  // tiles (5.7 and 6.3 us against 6.7 and 8.4), above in 128-row ones (37 and
-  // 59 us against 44 and 62 at 2^21 rows).
+  // Rows of 4-64 bytes: small tile-staged blocks, several per SM.  Doubling
+  // LDOS, us per step: real B = 1 / 2 / 4 / 8 on 1024^2 sites 23 / 28 / 34 / 54
+  // against 60 / 64 / 95 / 150 register-staged, on 181^2 3.1 / 3.5 / 4.3 / 5.4
+  // against 6.3 / 8.4 / 10 / 16; complex B = 1 / 2 / 4 / 8 on the 512^2 Rashba
+  // lattice 13 / 19 / 24 / 39 against 31 / 39 / 46 / 100.  Below 2^18 rows four
+  // and eight real sources are faster in 64-row tiles, above in 128-row ones
+  // (37 and 59 us against 44 and 62 at 2^21 rows).
+  // Wider rows: 8 real or 4 complex values per thread (B = 32 on 1024^2: 197
+  // us, directly gathered 152, against 267 and 247 with 4; complex B = 16 on
+  // the 512^2 Rashba lattice 72 against 97 with 2).  On the 2048^2 lattice real
+  // B = 64 / 128 / 256 take 1.43 / 3.01 / 5.71 ms against 2.90 / 4.79 / 11.8
+  // register-staged, on the 1024^2 Rashba lattice complex B = 32 / 64 / 128 /
+  // 256 0.55 / 1.09 / 2.14 / 4.27 against 1.25 / 1.94 / 3.33 / 8.28.  Without
+  // the dots more blocks fit: real B = 64 324 against 331 us on 1024^2, complex
+  // B = 128 514 against 532 on 512^2.
   const bool small = N != 0 && N <= (1u << 18);
   if (real) {
     if (B <= 1) return {1, 1, tiled(0, 256, 8, 3)};
@@ -175,8 +179,8 @@ Shape shape_for(int precision, uint32_t B, bool real = false, bool dots = false,
     if (B <= 4) return small ? Shape{1, 4, tiled(0, 64, 2, 8)} : Shape{1, 4, tiled(0, 128, 4, 6)};
     if (B <= 8) return small ? Shape{2, 4, tiled(0, 64, 4, 4)} : Shape{1, 8, tiled(51, 128, 4, 4)};
     if (B <= 16) return {2, 8, tiled(51, 64, 4, 4)};
-    if (B <= 32) return {8, 4, tiled(0, 64, 16, 1)};
-    if (B <= 64) return {8, 8, tiled(51, 64, 16, 1)};
+    if (B <= 32) return {4, 8, tiled(51, 64, 8, dots ? 2 : 3)};
+    if (B <= 64) return dots ? Shape{8, 8, tiled(51, 64, 16, 1)} : Shape{8, 8, tiled(51, 32, 8, 2)};
     if (B <= 128) return {16, 8, tiled(51, 16, 8, 2)};
     return {32, 8, tiled(51, 16, 16, 1)};
   }
@@ -184,10 +188,10 @@ Shape shape_for(int precision, uint32_t B, bool real = false, bool dots = false,
   if (B == 2) return {1, 2, tiled(0, 64, 2, 6)};
   if (B <= 4) return {2, 2, tiled(0, 64, 4, 6)};
   if (B <= 8) return {2, 4, tiled(0, 64, 4, 4)};
-  if (B <= 16) return {8, 2, tiled(0, 32, 8, 2)};
+  if (B <= 16) return {4, 4, tiled(0, 32, 4, 4)};
   if (B <= 32) return {8, 4, tiled(0, 32, 8, 2)};
   if (B <= 64) return {16, 4, tiled(0, 16, 8, 2)};
-  if (B <= 128) return {32, 4, tiled(0, 16, 16, 1)};
+  if (B <= 128) return dots ? Shape{32, 4, tiled(0, 16, 16, 1)} : Shape{32, 4, tiled(0, 8, 8, 2)};
   return {64, 4, tiled(0, 8, 16, 1)};
 }
 
@@ -260,7 +264,7 @@ const StepEntry *tuned_step(const tbtkkpm_matrix *m, int precision, bool dots, u
 const StepEntry *default_step(const tbtkkpm_matrix *m, int precision, bool dots, uint32_t B,
                               bool real64) {
   const bool real = real_mode(m, precision);
-  Shape s = shape_for(precision, B, real, dots, m->N);
+  Shape s = shape_for(precision, B, real, dots, m->N, m->widest_slice);
   if (real64) s = real64_shape_for(B);
   return find_step(step_class(precision, dots, real), s.tpr, s.vpt, s.minb);
 }
@@ -347,7 +351,8 @@ int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool 
         }
       }
     }
-    const Shape s = r64 ? shape_for(precision, B, false, dots, m->N) : register_shape_for(precision, B, real, dots);
+    const Shape s = r64 ? shape_for(precision, B, false, dots, m->N, m->widest_slice)
+                        : register_shape_for(precision, B, real, dots);
     fn = find_step(cls, s.tpr, s.vpt, s.minb);
   }
   return TBTKKPM_OK;

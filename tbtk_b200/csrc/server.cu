@@ -119,7 +119,8 @@ struct Model {
   uint32_t tcount = 0;
   bool dirty = true;
   DevBuf lane_mem;  // one allocation; the lane buffers above are views into it
-  // gather plans of the matrix by 2 * rows per tile + complex (null: none)
+  // gather plans of the matrix by 2 * rows per tile + complex, 1024 more for
+  // rows of at most 32 bytes (null: none)
   std::map<int, const TilePlan *> plans;
   void release_lanes() {
     for (DevBuf *b : {&vec[0], &vec[1], &dots, &mu, &mu_direct, &base, &laneM, &bitmap, &tlist,
@@ -148,7 +149,7 @@ struct RerunJob {
 // target bitmap and list (a row and an entry word for each of up to W
 // lane sites and W pair targets), pair moments.
 uint64_t lane_bytes(uint32_t N, uint32_t W, uint32_t Mmax, uint32_t ld, size_t esize) {
-  return 2ull * N * W * esize + 2ull * kDotsRing * W * sizeof(long long) +
+  return 2ull * (N + 3) * W * esize + 2ull * kDotsRing * W * sizeof(long long) +
          (uint64_t)W * Mmax * sizeof(double2) + (uint64_t)W * ld * sizeof(double2) +
          8ull * W + 4ull * ((N + 31) / 32) + 16ull * W + (uint64_t)W * Mmax * sizeof(double2);
 }
@@ -185,7 +186,8 @@ const MultiEntry *find_multi(int tpr, int vpt, int minb, bool real) {
 const TilePlan *model_plan(Model *m, uint32_t W, const MultiEntry *e, int *rc) {
   *rc = TBTKKPM_OK;
   if (!is_multi_tiled(e->minb) || (W * m->esize()) % 16 != 0) return nullptr;
-  const int R = multi_tiled_rows(e->minb), key = 2 * R + (m->real ? 0 : 1);
+  const bool narrow = W * m->esize() <= 32;
+  const int R = multi_tiled_rows(e->minb), key = (narrow ? 1024 : 0) + 2 * R + (m->real ? 0 : 1);
   auto it = m->plans.find(key);
   if (it != m->plans.end()) return it->second;
   // the first use builds it on the matrix handle (under its lock: the rerun
@@ -194,6 +196,14 @@ const TilePlan *model_plan(Model *m, uint32_t W, const MultiEntry *e, int *rc) {
   {
     std::lock_guard<std::mutex> lk(m->mat->lock);
     *rc = tile_plan(m->mat, R, !m->real, &p);
+    // Columns four at a time where that makes far fewer copies (a honeycomb's
+    // runs of two rows), as in fitting_plan of recursion.cu.  The copies may
+    // run three rows past a vector's end (make_resident).
+    if (!*rc && p && (narrow || p->nruns > (uint64_t)p->ntiles * (4 + R / 16))) {
+      const TilePlan *four = nullptr;
+      *rc = tile_plan(m->mat, R, !m->real, &four, false, 4);
+      if (!*rc && four && 2 * (uint64_t)four->nruns <= p->nruns) p = four;
+    }
   }
   if (*rc) return nullptr;
   m->plans[key] = p;
@@ -251,14 +261,14 @@ std::array<int, 3> default_config(uint32_t W, bool real) {
       case 4: return {1, 4, 164024};
       case 8: return {1, 8, 164024};
       case 16: return {2, 8, 164042};
-      case 32: return {8, 4, 164161};
+      case 32: return {4, 8, 164082};
       case 64: return {8, 8, 164161};
     }
   } else {
     switch (W) {
       case 4: return {1, 4, 164024};
       case 8: return {2, 4, 164042};
-      case 16: return {8, 2, 132082};
+      case 16: return {4, 4, 132042};
       case 32: return {8, 4, 132082};
       case 64: return {16, 4, 116082};
     }
@@ -359,8 +369,9 @@ int make_resident(tbtkkpm_server *s, Model *m) {
   constexpr int kViews = 10;
   DevBuf *views[kViews] = {&m->vec[0], &m->vec[1], &m->dots,   &m->mu,    &m->mu_direct,
                            &m->base,   &m->laneM,  &m->bitmap, &m->tlist, &m->pmu};
-  const size_t sizes[kViews] = {es * (size_t)N * W,
-                                es * (size_t)N * W,
+  // the staged copies may run three rows past a vector's end (model_plan)
+  const size_t sizes[kViews] = {es * ((size_t)N + 3) * W,
+                                es * ((size_t)N + 3) * W,
                                 2 * kDotsRing * sizeof(long long) * W,
                                 sizeof(double2) * (size_t)W * s->Mmax,
                                 sizeof(double2) * (size_t)W * s->ld,
@@ -1802,8 +1813,8 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
   const size_t es = probe->esize();
   DevBuf vec[2], dots, mu, mud, base, laneM, bitmap, tlist, dm, dh, tmap, tdesc, truns;
   int rc;
-  if ((rc = vec[0].reserve(es * (size_t)N * W)) ||
-      (rc = vec[1].reserve(es * (size_t)N * W)) ||
+  if ((rc = vec[0].reserve(es * ((size_t)N + 3) * W)) ||
+      (rc = vec[1].reserve(es * ((size_t)N + 3) * W)) ||
       (rc = dots.reserve(2 * kDotsRing * sizeof(long long) * W)) || (rc = mu.reserve(sizeof(double2) * W * Mp)) ||
       (rc = mud.reserve(sizeof(double2) * W * ldp)) || (rc = base.reserve(4 * W)) ||
       (rc = laneM.reserve(4 * W)) || (rc = bitmap.reserve(4 * (size_t)((N + 31) / 32))) ||
