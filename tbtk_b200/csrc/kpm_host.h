@@ -38,13 +38,34 @@ struct PhaseTimer {
   void destroy();
 };
 
-// A grow-only device allocation.
+// A grow-only device allocation (on the current device).
 struct DevBuf {
   void *ptr = nullptr;
   size_t cap = 0;
   int reserve(size_t n);
-  void release();
+  // Frees it, which waits for the device.  With `idle`, that no work on the
+  // buffer is in flight on any stream, the block may go to the cache that
+  // reserve() takes from first.
+  void release(bool idle = false);
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
+};
+
+// Counts a handle (matrix, table, server) for the block cache, which is
+// emptied when the last one goes.
+void cache_handle_added();
+void cache_handle_removed();
+
+// Buffers of one function's work on stream `st`, recycled at its end after
+// the stream has passed.
+template <int N> struct ScratchBufs {
+  cudaStream_t st;
+  DevBuf b[N];
+  explicit ScratchBufs(cudaStream_t s) : st(s) {}
+  ScratchBufs(const ScratchBufs &) = delete;
+  ~ScratchBufs() {
+    const bool idle = cudaStreamSynchronize(st) == cudaSuccess;
+    for (DevBuf &x : b) x.release(idle);
+  }
 };
 
 // Makes `dev` current for the scope and restores the previous device.
@@ -69,10 +90,10 @@ struct Workspace {
   DevBuf col_out;     // [Bp] output slot of each batch column (doubling runs)
   DevBuf err;         // device flag of a bounded wait that ran out
   DevBuf head, head_jobs, head_res;  // FP64 head of doubling runs (scratch, jobs, results)
-  void release() {
+  void release(bool idle) {
     for (DevBuf *b : {&vec[0], &vec[1], &bitmap, &tgt, &from, &mu, &damp, &out, &mu_direct,
                       &dots, &col_out, &err, &head, &head_jobs, &head_res})
-      b->release();
+      b->release(idle);
   }
 };
 
@@ -102,11 +123,8 @@ struct TilePlanStore {
   bool ok = false;
   TilePlan plan{};
   DevBuf hdr, runs, eslot, eval;
-  void release() {
-    hdr.release();
-    runs.release();
-    eslot.release();
-    eval.release();
+  void release(bool idle) {
+    for (DevBuf *b : {&hdr, &runs, &eslot, &eval}) b->release(idle);
   }
 };
 
@@ -154,17 +172,12 @@ struct tbtkkpm_matrix {
   // key 2048*(unit - 1) + 1024*pairs + 2*R + complex
   std::map<int, tbtkkpm::TilePlanStore> plans;
   std::mutex lock;
-  void release_all() {
-    for (auto &p : plans) p.second.release();
+  // `idle`: the handle's stream has passed its last work
+  void release_all(bool idle) {
+    for (auto &p : plans) p.second.release(idle);
     plans.clear();
-    rowptr.release();
-    col.release();
-    val2.release();
-    slice_ptr.release();
-    scol.release();
-    sval.release();
-    sreal.release();
-    ws.release();
+    for (tbtkkpm::DevBuf *b : {&rowptr, &col, &val2, &slice_ptr, &scol, &sval, &sreal}) b->release(idle);
+    ws.release(idle);
     timer.destroy();
   }
 };

@@ -881,6 +881,7 @@ static int table_alloc(uint32_t M, uint32_t E, tbtkkpm_table **out, bool with_ta
     delete t;
     return cuda_fail(e, "cudaStreamCreate");
   }
+  cache_handle_added();
   int rc = with_table ? t->table.reserve(sizeof(double2) * (size_t)M * E) : TBTKKPM_OK;
   if (rc) {
     tbtkkpm_table_destroy(t);
@@ -919,7 +920,7 @@ extern "C" int tbtkkpm_table_create(uint32_t M, const double *energies, uint32_t
                                                                      t->table.as<double2>());
   count_launches(1);
   cudaError_t e = cudaStreamSynchronize(t->stream);
-  en.release();
+  en.release(e == cudaSuccess);
   if (e != cudaSuccess) {
     tbtkkpm_table_destroy(t);
     return cuda_fail(e, "table_create");
@@ -1048,15 +1049,12 @@ extern "C" int tbtkkpm_table_destroy(tbtkkpm_table *t) {
   if (!t) return TBTKKPM_OK;
   {
     DeviceGuard g(t->device);
-    if (t->stream) cudaStreamSynchronize(t->stream);
-    t->table.release();
-    t->energies.release();
-    t->twiddle.release();
-    t->mu.release();
-    t->out.release();
+    const bool idle = !t->stream || cudaStreamSynchronize(t->stream) == cudaSuccess;
+    for (DevBuf *b : {&t->table, &t->energies, &t->twiddle, &t->mu, &t->out}) b->release(idle);
     if (t->stream) cudaStreamDestroy(t->stream);
   }
   delete t;
+  cache_handle_removed();
   return TBTKKPM_OK;
 }
 

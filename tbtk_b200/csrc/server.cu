@@ -1811,7 +1811,11 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
   const uint32_t W = width, N = probe->N, Mp = 2 * probe_steps + 2, ldp = Mp / 2 + 1;
   const bool real = probe->real;  // the class of the probe model is tuned
   const size_t es = probe->esize();
-  DevBuf vec[2], dots, mu, mud, base, laneM, bitmap, tlist, dm, dh, tmap, tdesc, truns;
+  ScratchBufs<15> scratch(st);
+  DevBuf *vec = scratch.b;
+  DevBuf &dots = vec[2], &mu = vec[3], &mud = vec[4], &base = vec[5], &laneM = vec[6],
+         &bitmap = vec[7], &tlist = vec[8], &dm = vec[9], &dh = vec[10], &tmap = vec[11],
+         &tdesc = vec[12], &truns = vec[13], &dj = vec[14];
   int rc;
   if ((rc = vec[0].reserve(es * ((size_t)N + 3) * W)) ||
       (rc = vec[1].reserve(es * ((size_t)N + 3) * W)) ||
@@ -1838,7 +1842,6 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
     tl[W + i] = t[i].second;
   }
   cudaError_t e;
-  DevBuf dj;
   if ((rc = dj.reserve(sizeof(MultiJoin) * W))) return rc;
   if ((e = cudaMemsetAsync(vec[1].ptr, 0, es * (size_t)N * W, st)) ||
       (e = cudaMemsetAsync(dots.ptr, 0, 2 * kDotsRing * sizeof(long long) * W, st)) ||
@@ -2045,7 +2048,7 @@ extern "C" int tbtkkpm_server_destroy(tbtkkpm_server *s) {
     for (DevBuf *b : {&s->d_models, &s->d_hdr, &s->d_joins, &s->d_done, &s->d_pairs, &s->d_stage,
                       &s->d_damp, &s->d_tiles, &s->d_tdesc, &s->d_truns, &s->d_err, &s->d_step})
       b->release();
-    s->head_ws.release();
+    s->head_ws.release(false);
     s->d_res.release();
     if (s->h_res) cudaFreeHost(s->h_res);
     if (s->h_err) cudaFreeHost(s->h_err);

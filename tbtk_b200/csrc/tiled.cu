@@ -64,7 +64,9 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, T
   cudaStream_t st = m->stream;
   const uint32_t ntiles = (m->N + R - 1) / R;
   const unsigned grid = (unsigned)std::min<uint64_t>(ntiles, (uint64_t)sm_count(m->device) * 8);
-  DevBuf tw, truns, tuniq, ent, run, flags, tmp;
+  ScratchBufs<7> scratch(st);
+  DevBuf &tw = scratch.b[0], &truns = scratch.b[1], &tuniq = scratch.b[2], &ent = scratch.b[3],
+         &run = scratch.b[4], &flags = scratch.b[5], &tmp = scratch.b[6];
   int rc;
   if ((rc = tw.reserve(4 * ((size_t)ntiles + 1))) || (rc = truns.reserve(4 * ((size_t)ntiles + 1))) ||
       (rc = tuniq.reserve(4 * ((size_t)ntiles + 1))) || (rc = ent.reserve(4 * ((size_t)ntiles + 1))) ||
@@ -163,7 +165,7 @@ int tile_plan(tbtkkpm_matrix *m, int R, bool cplx, const TilePlan **out, bool pa
     TilePlanStore &p = m->plans[key];
     int rc = build_plan(m, R, cplx, pairs, unit, p);
     if (rc) {
-      p.release();
+      p.release(false);
       m->plans.erase(key);
       return rc;
     }
