@@ -256,6 +256,9 @@ TBTKKPM_API int tbtkkpm_ldos(
  * CUDA events on the handle's stream, and keeps the fastest for later calls
  * on this handle.  ldos != 0 tunes the kernels tbtkkpm_ldos_sites uses (the
  * dot-product variant at TBTKKPM_MIXED), 0 those of the moment calls.
+ * A small matrix whose recursion runs on chip by default keeps that when it is
+ * faster than every configuration; the outputs are the fastest
+ * configuration's all the same.
  * Outputs (may be NULL): the chosen configuration and its ms per step.
  * tbtkkpm_matrix_set_config installs a known choice without timing.
  * (No reference counterpart.) */
@@ -564,8 +567,8 @@ TBTKKPM_API int tbtkkpm_server_set_table_free(tbtkkpm_server *s, int enable);
 /* enable = 1 (the default): a tick whose steps are shorter than their launches
  * (many lane classes of small models) replays a CUDA graph of one step of
  * every lane class, captured when the tick starts (a device counter gives each
- * replay its step); enable = 0 launches every kernel of every step directly.  A capture that fails turns graphs off for the server.
- * Results do not depend on it.  (No reference counterpart.) */
+ * replay its step); enable = 0 launches every kernel of every step directly.
+ * A capture that fails turns graphs off for the server.  Results do not depend on it.  (No reference counterpart.) */
 TBTKKPM_API int tbtkkpm_server_set_graphs(tbtkkpm_server *s, int enable);
 
 /* enable = 1 (the default): a model steps at the narrowest width (a power

@@ -161,8 +161,8 @@ REAL_DOTS_OPTS = {
 }
 # Tile-staged steps (kpm_tiled.cuh): (threads per row, values per thread)
 # shapes with (rows per tile, consumer warps, blocks per SM, widening split
-# CV) variants.  Rows of real floats are staged with 16-byte chunks, so a
-# thread holds 4 or 8 values.  On the 2048^2 lattice at 64 columns (8, 8)
+# CV) variants.  Rows under the 16 bytes of a bulk copy (1 or 2 real values,
+# 1 complex) are staged in units of four columns.  On the 2048^2 lattice at 64 columns (8, 8)
 # with 64-row tiles and 16 consumer warps took 1.46 ms per step, 32-row
 # tiles at two blocks per SM 1.60 ms, both with every widening on the XU
 # pipe (69% busy in the ncu capture); CV moves widenings to the integer pipe.
@@ -223,8 +223,8 @@ TILED_CPLX = {
 # warps, blocks per SM).  Rows of 16-byte values: B = 16 / 32 / 64 / 128
 # take 256 B / 512 B / 1 KB / 2 KB per row.
 TILED_FP64 = {
-    (1, 1): [(64, 2, 8), (64, 2, 6), (64, 2, 4), (128, 4, 4)],
-    (2, 1): [(64, 4, 6), (64, 4, 4), (128, 8, 3)],
+    (1, 1): [(64, 2, 8), (64, 2, 6), (32, 1, 8), (64, 2, 4), (128, 4, 4)],
+    (2, 1): [(64, 4, 6), (64, 4, 4), (32, 2, 8), (128, 8, 3)],
     (4, 1): [(64, 8, 4), (64, 8, 3), (64, 8, 2), (32, 4, 6)],
     (8, 1): [(64, 16, 2), (32, 8, 4), (64, 8, 3)],
     (16, 1): [(32, 8, 2), (64, 16, 1)],

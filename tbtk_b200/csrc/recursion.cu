@@ -53,8 +53,7 @@ bool real64_mode(const tbtkkpm_matrix *m, int precision) {
 }
 
 // The register-staged shape of a batch (kpm_step / kpm_step_real): the
-// fallback of the tile-staged defaults below, and the default of widths the
-// tile-staged steps do not serve.
+// fallback of the tile-staged defaults below.
 Shape register_shape_for(int precision, uint32_t B, bool real, bool dots) {
   if (real) {
     // a thread per row up to 8 values: it prefetches all of the next row's
