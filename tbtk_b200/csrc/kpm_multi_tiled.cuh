@@ -255,9 +255,12 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
     long long s_nn[VPT], s_np[VPT];
 #pragma unroll
     for (int j = 0; j < VPT; j++) s_nn[j] = s_np[j] = 0;
-    // the warp's sums over threads of the same columns, one atomic per
-    // column and warp (warp-uniform: the warp's threads share the tile)
-    auto flush = [&]() {
+    auto add = [&](uint32_t c, long long v) {
+      if (v) atomicAdd(reinterpret_cast<unsigned long long *>(t_dots + c), (unsigned long long)v);
+    };
+    // the warp's sums over threads of the same columns, put(c, sum) by one lane
+    // (warp-uniform: the warp's threads share the tile)
+    auto flush = [&](auto put) {
 #pragma unroll
       for (int j = 0; j < VPT; j++) {
         long long a = s_nn[j], b = s_np[j];
@@ -268,8 +271,8 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
         }
         if (lane < TPR) {
           const uint32_t c = Pk::col_of(sub, j);
-          if (a) atomicAdd(reinterpret_cast<unsigned long long *>(t_dots + c), (unsigned long long)a);
-          if (b) atomicAdd(reinterpret_cast<unsigned long long *>(t_dots + W + c), (unsigned long long)b);
+          put(c, a);
+          put(W + c, b);
         }
         s_nn[j] = s_np[j] = 0;
       }
@@ -283,7 +286,7 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
       }
       const MultiStageMeta mt = smeta[s];
       if (mt.model != cq) {
-        if (cq != kPad) flush();
+        if (cq != kPad) flush(add);
         cq = mt.model;
         t_dots = mt.dots;
         m_y = static_cast<E *>(mt.y);
@@ -433,7 +436,23 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
-    if (cq != kPad) flush();
+    // The last sums go over the block's warps through the ring (every warp has
+    // used its last stage; after a wait that ran out the step's results are
+    // dropped), then one atomic per column and block: atomics on the same few
+    // addresses go one by one in L2 (16 lanes of a 74k-row model: 11.5 us a
+    // step, with one atomic per column and warp 27.5).
+    static_assert(R >= CW, "the warps' sums fit two stages of the ring");
+    constexpr uint32_t kThreads = CW * 32;
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+    long long *red = reinterpret_cast<long long *>(ring);
+    flush([&](uint32_t c, long long v) { red[(uint32_t)(warp - 1) * 2 * W + c] = v; });
+    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+    for (uint32_t c = (uint32_t)ct; c < 2 * W; c += kThreads) {
+      long long v = 0;
+#pragma unroll
+      for (int u = 0; u < CW; u++) v += red[(uint32_t)u * 2 * W + c];
+      add(c, v);
+    }
     if (failed && lane == 0) atomicExch(err, kErrTimeout);
   }
 }

@@ -446,6 +446,21 @@ struct JoinRef {
   Request *r;
 };
 
+// Consecutive tiles that a block of a tile-staged launch takes at a time.  The
+// blocks get equal shares, in one run for up to 15 tiles a block and up to four
+// for more (models of one class differ in tile cost), of at most 32 tiles; a
+// run changes model rarely.  Runs of 8-32 tiles left most blocks idle while a
+// few small models were under way and gave a block up to 8 tiles more than
+// another: alone, 1056 rows at 8 lanes took 16.6 us a step (6.4 now), 5040 at
+// 1 lane of 16 13.0 (6.3), 131k complex rows at one lane 20.9 (13.7).
+uint32_t tiles_in_a_row(uint32_t tiles, int variant, int device) {
+  if (!is_multi_tiled(variant)) return kRun;
+  const uint32_t grid = std::max(1u, (uint32_t)multi_tiled_bps(variant) * (uint32_t)sm_count(device));
+  const uint32_t share = std::max(1u, (tiles + grid - 1) / grid);
+  const uint32_t rounds = std::max(std::min(std::max(share / kRun, 1u), 4u), (share + 31) / 32);
+  return std::max(1u, (tiles + grid * rounds - 1) / (grid * rounds));
+}
+
 // A change of a model's step width at a step boundary: its two lane
 // buffers are restrided in place (run_relayouts) before the joins run.
 struct Relayout {
@@ -842,13 +857,7 @@ int run_tick(tbtkkpm_server *s, const std::vector<ClassPlan> &plans, uint32_t ns
   tiles = runs = 0;
   for (const ClassPlan &cp : plans) {
     all.insert(all.end(), cp.models.begin(), cp.models.end());
-    // tile-staged launches: runs of 8-32 tiles per block, long enough that
-    // a block rarely changes model, short enough that every block has work
-    uint32_t run = kRun;
-    if (is_multi_tiled(cp.entry->minb)) {
-      const uint32_t grid = (uint32_t)multi_tiled_bps(cp.entry->minb) * (uint32_t)sm_count(s->device);
-      run = std::max(kRun, std::min(32u, cp.total_tiles / std::max(4 * grid, 1u)));
-    }
+    const uint32_t run = tiles_in_a_row(cp.total_tiles, cp.entry->minb, s->device);
     hdr.push_back({(uint32_t)cp.models.size(), cp.total_tiles, s->n_global,
                    s->d_tiles.as<uint32_t>() + tiles, s->d_tdesc.as<uint4>() + kDescWords * tiles,
                    s->d_truns.as<uint2>() + runs, run, graph ? s->d_step.as<int32_t>() : nullptr});
@@ -1907,11 +1916,7 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
         (rc = tdesc.reserve(16 * kDescWords * (size_t)d.ntiles)) ||
         (rc = truns.reserve(8 * (size_t)std::max(d.p_nruns, 1u))))
       break;
-    uint32_t run = kRun;
-    if (plan) {
-      const uint32_t grid = (uint32_t)multi_tiled_bps(en.minb) * (uint32_t)sm_count(s->device);
-      run = std::max(kRun, std::min(32u, d.ntiles / std::max(4 * grid, 1u)));
-    }
+    const uint32_t run = tiles_in_a_row(d.ntiles, en.minb, s->device);
     MultiHeader h{1, d.ntiles, n, tmap.as<uint32_t>(), tdesc.as<uint4>(), truns.as<uint2>(), run};
     // parity of the buffers follows the global step, so the probe keeps
     // counting across configurations
