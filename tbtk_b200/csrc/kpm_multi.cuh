@@ -171,6 +171,14 @@ inline void lane_relayout_ranges(uint32_t N, uint32_t W, uint32_t W2,
 // so it changes model (and flushes its sums) at most once per run.
 constexpr uint32_t kRun = 8;
 
+// The same for the register-staged steps: shorter runs at one and two lanes
+// while there are fewer than kRun tiles per block, else most blocks are idle
+// (39k rows at one lane: 18.6 us a step with runs of 8, 8.0 so).  Wider steps
+// keep kRun: each block's atomics on the lanes' few sums cost them more.
+__device__ __forceinline__ uint32_t register_run(uint32_t tiles, uint32_t W) {
+  return W > 2 ? kRun : max(1u, min(kRun, (tiles + gridDim.x - 1) / gridDim.x));
+}
+
 // Fills the tile -> model map of a launch: one block per model.
 static __global__ void kpm_multi_tilemap(const MultiModel *__restrict__ models,
                                          const MultiHeader *__restrict__ hdr, uint32_t *tile_model) {
@@ -222,6 +230,7 @@ kpm_multi_step(const MultiModel *__restrict__ models, const MultiHeader *__restr
   const int grp = threadIdx.x / TPR;
   const unsigned mask = 0xffffffffu;
   const uint32_t nmodels = hdr->nmodels, total = hdr->total_tiles;
+  const uint32_t run = register_run(total, W);
   const uint32_t *__restrict__ tile_model = hdr->tile_model;
   const int32_t n = multi_step_index(hdr, step_offset);
   if (nmodels == 0) return;
@@ -272,13 +281,13 @@ kpm_multi_step(const MultiModel *__restrict__ models, const MultiHeader *__restr
   // the tile after w in this block's order
   auto next_tile = [&](uint32_t w) -> uint32_t {
     const uint32_t nw = w + 1;
-    if (nw % kRun != 0) return nw;
-    return (w / kRun + gridDim.x) * kRun;
+    if (nw % run != 0) return nw;
+    return (w / run + gridDim.x) * run;
   };
 
   RowFetch<V, AR, TPR, VPT, PF> cur, nxt;
   uint32_t cur_model = 0, nxt_model = 0;
-  uint32_t w = blockIdx.x * kRun;
+  uint32_t w = blockIdx.x * run;
   if (w < total) {
     const RowBounds b0 = bounds_of(w, cur_model);
     fetch(w, cur_model, b0, cur);

@@ -23,6 +23,7 @@ kpm_multi_step_real(const MultiModel *__restrict__ models, const MultiHeader *__
   const int grp = threadIdx.x / TPR;
   const unsigned mask = 0xffffffffu;
   const uint32_t nmodels = hdr->nmodels, total = hdr->total_tiles;
+  const uint32_t run = register_run(total, W);
   const uint32_t *__restrict__ tile_model = hdr->tile_model;
   const int32_t n = multi_step_index(hdr, step_offset);
   if (nmodels == 0) return;
@@ -70,13 +71,13 @@ kpm_multi_step_real(const MultiModel *__restrict__ models, const MultiHeader *__
   };
   auto next_tile = [&](uint32_t t) -> uint32_t {
     const uint32_t nt = t + 1;
-    if (nt % kRun != 0) return nt;
-    return (t / kRun + gridDim.x) * kRun;
+    if (nt % run != 0) return nt;
+    return (t / run + gridDim.x) * run;
   };
 
   RRowFetch<TPR, VPT, PF> cur, nxt;
   uint32_t cur_model = 0, nxt_model = 0;
-  uint32_t w = blockIdx.x * kRun;
+  uint32_t w = blockIdx.x * run;
   if (w < total) {
     const RowBounds b0 = bounds_of(w, cur_model);
     fetch(w, cur_model, b0, cur);
