@@ -215,7 +215,7 @@ def step_bytes(p, B, s_vec, s_val=16):
     column indices, row pointers) and three vector passes per source
     (gather of j_n counted once, read of j_{n-1}, write of j_{n+1}).
     s_vec/s_val: bytes per vector element / stored value (complex128 16/16,
-    complex64 8/16, real vectors of a real matrix 4/8)."""
+    complex64 8/16, real vectors of a real matrix 4/8, in FP64 8/8)."""
     return p.nnz * (s_val + 4) + 4 * (p.N + 1) + 3 * p.N * B * s_vec
 
 
@@ -581,6 +581,8 @@ def ours(args, world, rank, local):
     value = solves / (total_ms / 1e3)
     avg_step_ms = rec_ms / max(rec_launches, 1)
     bstep = step_bytes(p, B, 4, 8) if real_vectors else step_bytes(p, B, 8)
+    fp64_step = step_bytes(p, B, 8, 8) if real_vectors else step_bytes(p, B, 16)
+    fp64_kind = "real double" if real_vectors else "complex128"
     achieved = bstep / (avg_step_ms / 1e3) / 1e9
     vec_kind = "real float" if real_vectors else "complex64"
     traffic_row = traffic_per_row(vec_kind, B, tuned_mixed)
@@ -615,14 +617,12 @@ def ours(args, world, rank, local):
             "value": B / (fp64_ms / 1e3), "unit": "LDOS solves/s", "ms_per_call": fp64_ms,
             "sites": B,
             "step_ms": fp64_rec / max(fp64_launches, 1),
-            "roofline": {"achieved_GBps": step_bytes(p, B, 16) / (fp64_rec / max(fp64_launches, 1)
-                                                                  / 1e3) / 1e9,
-                         "frac": step_bytes(p, B, 16) / (fp64_rec / max(fp64_launches, 1) / 1e3)
-                                 / 1e9 / peak,
-                         "bytes_per_launch": step_bytes(p, B, 16)},
+            "roofline": {"achieved_GBps": fp64_step / (fp64_rec / max(fp64_launches, 1) / 1e3) / 1e9,
+                         "frac": fp64_step / (fp64_rec / max(fp64_launches, 1) / 1e3) / 1e9 / peak,
+                         "bytes_per_launch": fp64_step},
             "bit_identical_to_single_vector": all(np.array_equal(ref_all[i], plain_out[i])
                                                   for i in range(len(plain_out))),
-            "note": ("the same sites in one batched FP64 recursion on complex128 vectors, M-1 "
+            "note": (f"the same sites in one batched FP64 recursion on {fp64_kind} vectors, M-1 "
                      "steps in the reference's operation order (TBTK's default precision through "
                      "the seam); its LDOS is the reference for ldos_rel_err_vs_fp64")},
         "speedup_vs_plain_fp64": (value / world) / plain_rate if plain_rate else None,
@@ -633,7 +633,7 @@ def ours(args, world, rank, local):
             "plain_step_ms": plain_rec / max(plain_launches, 1),
             "batched_step_ms_per_site": avg_step_ms / B,
             "note": ("doubling: M-1 single-vector steps against M/2 doubling steps; the other "
-                     "factor compares one complex128 single-vector step with one site's share of "
+                     f"factor compares one {fp64_kind} single-vector step with one site's share of "
                      "the batched step (real float vectors for this real model); their product "
                      "is the speed-up before the energy sums and the FP64 head")},
         "ldos_rel_err_vs_fp64": max(errs) if errs else None,

@@ -88,8 +88,8 @@ def main():
         mat.set_real(False)
     if a.batch_width:
         mat.set_batch_width(prec, a.batch_width)
-    real = prec != kpm.FP64 and mat.real()[1]
-    s_vec = 16 if prec == kpm.FP64 else (4 if real else 8)
+    real = mat.real()[1]
+    s_vec = (16 if prec == kpm.FP64 else 8) // (2 if real else 1)
     # a call runs its sites in batches of the handle's width, each batch the
     # same number of steps: the mean algorithmic bytes of one launch
     width = mat.batch_width(prec, ldos=True)
