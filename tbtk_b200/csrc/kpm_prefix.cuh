@@ -140,7 +140,7 @@ __device__ __forceinline__ uint32_t prefix_enter(uint32_t *key, uint32_t row) {
 // j_q and j_{q-1} into its column of the two recursion buffers (zero
 // elsewhere beforehand), rounded once to FP32.
 template <bool REAL>
-__global__ void __launch_bounds__(kPrefixBlock)
+__global__ void __launch_bounds__(kPrefixBlock, 1)
 kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, PrefixResult *res) {
   using V = PrefixVec<REAL>;
   using T = typename V::T;
@@ -177,19 +177,12 @@ kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, PrefixResult *res)
   uint32_t f0 = 0, f1 = 1, q = 0;
   double2 mu1 = make_double2(0.0, 0.0);
   for (uint32_t n = 0; n < J.steps; n++) {
-    // Rows of the next ball: neighbours of the last step's new rows, a thread
-    // per (row, entry).  A new row gets the next local index and zero values
-    // in all three vectors; a warp takes the indices of its lanes' new rows at
-    // once.  Past kPrefixRows, or with no free slot, s_over is set instead.
-    const uint32_t enter = (f1 - f0) * J.width;
-    for (uint32_t b = 32 * warp; b < enter; b += kPrefixBlock) {
-      const uint32_t t = b + lane, i = f0 + t / J.width, k = t % J.width;
-      uint32_t c = kPad;
-      if (t < enter) {
-        const uint32_t r = rows[i], s = r >> 5;
-        const uint32_t cb = __ldg(J.slice_ptr + s), ce = __ldg(J.slice_ptr + s + 1);
-        if (cb + k < ce) c = __ldg(J.scol + (uint64_t)(cb + k) * 32 + (r & 31));
-      }
+    // Rows of the next ball: neighbours of the last step's new rows.  A new
+    // row gets the next local index and zero values in all three vectors; a
+    // warp takes the indices of its lanes' new rows at once.  Past kPrefixRows,
+    // or with no free slot, s_over is set instead, and the step, which is then
+    // dropped, ends at a warp's next look at it, before the table is full.
+    auto enter = [&](uint32_t c) {  // a column per lane, or kPad
       const uint32_t at = c != kPad ? prefix_enter(key, c) : kPrefixSlots;
       if (at > kPrefixSlots) s_over = 1;
       const uint32_t fresh = __ballot_sync(0xffffffffu, at < kPrefixSlots);
@@ -203,6 +196,36 @@ kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, PrefixResult *res)
           v[id] = v[kPrefixRows + id] = v[2 * kPrefixRows + id] = V::zero();
         } else {
           s_over = 1;
+        }
+      }
+    };
+    auto over = [&]() { return __any_sync(0xffffffffu, *(volatile uint32_t *)&s_over != 0); };
+    if (listed) {
+      // a thread per (row, entry): at most kPrefixRows * kPrefixWidth of them
+      const uint32_t count = (f1 - f0) * J.width;
+      for (uint32_t b = 32 * warp; b < count && !over(); b += kPrefixBlock) {
+        const uint32_t t = b + lane, i = f0 + t / J.width, k = t % J.width;
+        uint32_t c = kPad;
+        if (t < count) {
+          const uint32_t r = rows[i], s = r >> 5;
+          const uint32_t cb = __ldg(J.slice_ptr + s), ce = __ldg(J.slice_ptr + s + 1);
+          if (cb + k < ce) c = __ldg(J.scol + (uint64_t)(cb + k) * 32 + (r & 31));
+        }
+        enter(c);
+      }
+    } else {
+      // A warp per row up to the row's own last entry: one long row of the
+      // matrix makes J.width thousands where a row of the ball has a few (a
+      // row of 5000 entries outside the ball: walking J.width positions per
+      // row took 3.7 ms a head, this 0.41).
+      for (uint32_t i = f0 + warp; i < f1; i += kPrefixBlock / 32) {
+        const uint32_t r = rows[i], s = r >> 5;
+        const uint32_t cb = __ldg(J.slice_ptr + s), ce = __ldg(J.slice_ptr + s + 1);
+        for (uint32_t k = cb; k < ce && !over(); k += 32) {
+          const uint32_t c =
+              lane < ce - k ? __ldg(J.scol + ((uint64_t)k + lane) * 32 + (r & 31)) : kPad;
+          enter(c);
+          if (__any_sync(0xffffffffu, c == kPad)) break;
         }
       }
     }
@@ -258,7 +281,7 @@ kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, PrefixResult *res)
         for (uint32_t k = cb; k < ce; k++) {
           const uint64_t slot = (uint64_t)k * 32 + l;
           const uint32_t c = __ldg(J.scol + slot);
-          if (c == kPad) continue;
+          if (c == kPad) break;  // padding ends a row
           const int j = prefix_find(key, index, c);
           if (j >= 0) acc = V::mac(acc, V::value(__ldg(J.sval + slot)), x[j]);
         }
