@@ -318,8 +318,10 @@ TBTKKPM_API int tbtkkpm_matrix_set_fp64_head(tbtkkpm_matrix *m, uint32_t steps);
  * TBTKKPM_WAIT_DEFAULT).  A wait that runs out ends the step early, its
  * issued copies are waited for with the default bound, and the call returns
  * TBTKKPM_ERR_TIMEOUT; the handle stays usable.  polls = 0 makes every
- * such wait give up at once, which tests that path.  (No reference
- * counterpart: the reference's device waits are unbounded,
+ * such wait give up at once, which tests that path.  A handle with a bound
+ * of its own takes launched steps where a small matrix's recursion would run
+ * on chip, without such waits.  (No reference counterpart: the reference's
+ * device waits are unbounded,
  * Lib/src/Utilities/GPUResourceManager.cpp:52-73.) */
 #define TBTKKPM_WAIT_DEFAULT 0xffffffffu
 TBTKKPM_API int tbtkkpm_matrix_set_wait_limit(tbtkkpm_matrix *m, uint32_t polls);

@@ -142,6 +142,8 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
                   const uint32_t *tcol, uint32_t T, ResidentPlan &out) {
   out = ResidentPlan{};
   if (m->nslices > kResMaxSlices || m->nslices == 0 || B == 0) return TBTKKPM_OK;
+  // a handle with a wait bound of its own runs the steps whose waits it bounds
+  if (m->wait_limit != TBTKKPM_WAIT_DEFAULT) return TBTKKPM_OK;
   if (m->host_slice_ptr.size() != (size_t)m->nslices + 1) {
     std::vector<uint32_t> sp((size_t)m->nslices + 1);
     cudaError_t e = cudaMemcpyAsync(sp.data(), m->slice_ptr.ptr, 4 * sp.size(), cudaMemcpyDeviceToHost,

@@ -1,0 +1,41 @@
+"""Which calls run on chip and which as launched steps: an on-chip run adds a
+handful of kernel launches, launched steps one and more each."""
+import numpy as np
+import pytest
+
+from test_resident import SCALE
+from tbtk_b200 import lattice as L
+
+pytestmark = pytest.mark.gpu
+
+M = 200  # 199 steps, or 100 with doubling
+
+
+def _launches(gpu, call):
+    n = gpu.kernel_launches()
+    call()
+    return gpu.kernel_launches() - n
+
+
+def _ldos_launches(gpu, m, sites, precision):
+    tab = gpu.Table.create(M, gpu.tbtk_range(-SCALE, SCALE, 20, False, False), SCALE)
+    return _launches(gpu, lambda: m.ldos_sites(tab, sites, 1e-3, precision))
+
+
+@pytest.mark.parametrize("alpha", [0.0, 0.3])
+def test_a_wait_bound_takes_launched_steps(gpu, alpha):
+    """A handle with a wait bound runs the steps that have such waits, by
+    default too; the bound of 0 gives up at once."""
+    csr = L.square(24, 20, t=1.0, J=0.5, W=2.0, alpha=alpha, periodic=True, seed=5).csr()
+    sites = np.arange(64, dtype=np.uint32)
+    m = gpu.Matrix.from_csr(*csr, SCALE)
+    m.set_fp64_head(0)
+    assert _ldos_launches(gpu, m, sites, gpu.MIXED) < 20
+    m.set_wait_limit(0)
+    with pytest.raises(gpu.TBTKError) as e:
+        _ldos_launches(gpu, m, sites, gpu.MIXED)
+    assert e.value.status == gpu.ERR_TIMEOUT
+    m.set_wait_limit(1 << 24)
+    assert _ldos_launches(gpu, m, sites, gpu.MIXED) >= M // 2
+    m.set_wait_limit()
+    assert _ldos_launches(gpu, m, sites, gpu.MIXED) < 20
