@@ -3,7 +3,7 @@ handful of kernel launches, launched steps one and more each."""
 import numpy as np
 import pytest
 
-from test_resident import SCALE
+from test_resident import SCALE, _hermitian
 from tbtk_b200 import lattice as L
 
 pytestmark = pytest.mark.gpu
@@ -20,6 +20,19 @@ def _launches(gpu, call):
 def _ldos_launches(gpu, m, sites, precision):
     tab = gpu.Table.create(M, gpu.tbtk_range(-SCALE, SCALE, 20, False, False), SCALE)
     return _launches(gpu, lambda: m.ldos_sites(tab, sites, 1e-3, precision))
+
+
+@pytest.mark.parametrize("B", [1, 2, 12, 64, 128])
+@pytest.mark.parametrize("complex_", [False, True])
+@pytest.mark.parametrize("N", [1, 31, 100, 513, 1800])
+def test_small_matrices_run_on_chip(gpu, N, complex_, B):
+    """The sizes that test_resident compares with the step kernels."""
+    m = gpu.Matrix.from_csr(*_hermitian(N, 6, complex_, N), SCALE)
+    sites = (np.arange(B) * 5 % N).astype(np.uint32)
+    for p in (gpu.FP64, gpu.MIXED, gpu.MIXED_DIRECT):
+        assert _ldos_launches(gpu, m, sites, p) < 20, p
+    n = _launches(gpu, lambda: m.moments_batched(sites, sites, np.arange(B), M, 1e-3, gpu.FP64))
+    assert n < 20
 
 
 @pytest.mark.parametrize("alpha", [0.0, 0.3])
