@@ -307,22 +307,8 @@ kpm_resident(ResidentArgs R) {
   const uint32_t s0 = min(rank * R.spb, R.A.nslices), s1 = min(s0 + R.spb, R.A.nslices), ns = s1 - s0;
   const uint32_t cb0 = __ldg(R.A.slice_ptr + s0), nch = __ldg(R.A.slice_ptr + s1) - cb0;
   const uint32_t xbase = (uint32_t)__cvta_generic_to_shared(xs);
-  // the block's targets in this group, in row order; more than `cap` of them
-  // are stored step by step instead (staged false, first[] counts in R.tg)
   const uint32_t ta = target_first(R.tg, s0 * 32), tb = target_first(R.tg, s1 * 32);
-  if (threadIdx.x == 0) {
-    uint32_t nt = 0;
-    for (uint32_t t = ta; t < tb; t++) {
-      const uint32_t c = __ldg(R.tg.col + t) - c0;
-      if (c >= (uint32_t)COLS) continue;
-      if (nt < R.cap) {
-        tcol[nt] = c;
-        tout[nt] = __ldg(R.tg.out + t);
-      }
-      nt++;
-    }
-    s_nt = nt;
-  }
+  if (threadIdx.x == 0) s_nt = 0;
   // the block's rows of both vectors
   const V *gx = static_cast<const V *>(R.x), *gy = static_cast<const V *>(R.y);
   for (uint32_t i = threadIdx.x; i < rows + 4; i += blockDim.x) {
@@ -341,19 +327,47 @@ kpm_resident(ResidentArgs R) {
     if (i < rows) first[i] = kNoEntry;
   }
   __syncthreads();
+  // The block's targets in this group, and the first one of each row.  Up to
+  // `cap` of them are staged, in row order; more are stored step by step
+  // instead (staged false, first[] counts in R.tg).  All threads look: one
+  // alone took 0.1 us a target of the block's rows, whatever its column (2.6
+  // ms before 64 sources with 512 targets each could start).
+  for (uint32_t t = ta + threadIdx.x; t < tb; t += blockDim.x) {
+    if (__ldg(R.tg.col + t) - c0 >= (uint32_t)COLS) continue;
+    const uint32_t k = atomicAdd(&s_nt, 1u);
+    if (k < R.cap) tout[k] = t;
+    atomicMin(&first[__ldg(R.tg.row + t) - s0 * 32], t);
+  }
+  __syncthreads();
   const uint32_t nt = s_nt;
   const bool staged = nt <= R.cap;
-  if (threadIdx.x == 0) {
-    uint32_t k = 0;
-    for (uint32_t t = ta; t < tb; t++) {
-      if (__ldg(R.tg.col + t) - c0 >= (uint32_t)COLS) continue;
-      uint32_t &f = first[__ldg(R.tg.row + t) - s0 * 32];
-      if (f == kNoEntry) {
-        f = staged ? k : t;
-        if (staged) tcol[k] |= kTargetNew;
-      }
-      k++;
+  static_assert(kResTargets <= 64, "two targets per thread of a warp");
+  uint32_t mine[2], rank_of[2];
+  if (staged) {
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const uint32_t k = threadIdx.x + u * blockDim.x;
+      mine[u] = k < nt ? tout[k] : kNoEntry;
+      rank_of[u] = 0;
+      if (k < nt)
+        for (uint32_t j = 0; j < nt; j++) rank_of[u] += tout[j] < mine[u] ? 1u : 0u;
     }
+  }
+  __syncthreads();
+  if (staged) {
+    bool lead[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      lead[u] = false;
+      if (mine[u] == kNoEntry) continue;
+      lead[u] = first[__ldg(R.tg.row + mine[u]) - s0 * 32] == mine[u];
+      tcol[rank_of[u]] = (__ldg(R.tg.col + mine[u]) - c0) | (lead[u] ? kTargetNew : 0u);
+      tout[rank_of[u]] = __ldg(R.tg.out + mine[u]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+      if (lead[u]) first[__ldg(R.tg.row + mine[u]) - s0 * 32] = rank_of[u];
   }
   uint32_t radr[REG ? kResRegs : 1];
   Val rval[REG ? kResRegs : 1];
@@ -444,8 +458,10 @@ kpm_resident(ResidentArgs R) {
             }
           } else {
             const uint32_t r = s0 * 32 + i;
+            // a row's targets are in column order
             for (uint32_t t = f; t < R.tg.count && __ldg(R.tg.row + t) == r; t++) {
               const uint32_t c = __ldg(R.tg.col + t) - c0;
+              if (c >= (uint32_t)COLS) break;
 #pragma unroll
               for (int j = 0; j < COLS; j++)
                 if (c == (uint32_t)j)
