@@ -5,6 +5,7 @@
 #include "kpm_resident.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 namespace tbtkkpm {
@@ -64,6 +65,8 @@ static bool shape_resident(const tbtkkpm_matrix *m, const uint32_t *trow, const 
     p.cap = std::max(p.cap, ++count[(size_t)(trow[t] / (p.spb * 32)) * p.groups + tcol[t] / p.cols]);
   if (p.cap > kResTargets) p.cap = 0;
   p.reg = p.spb <= p.warps && m->widest_slice <= (uint32_t)kResRegs;
+  // (also keeps the layout's 32-bit offsets from wrapping)
+  if (!p.reg && (uint64_t)p.chunks * 32 * (value_size(p.kind) + 4) > kResSmem) return false;
   p.smem = resident_layout(p.spb, p.chunks, p.cap, p.warps, p.cols, (uint32_t)vec_elem_size(p.kind),
                            (uint32_t)value_size(p.kind), p.reg, p.dots).bytes;
   return p.smem <= kResSmem;
@@ -112,30 +115,47 @@ static uint32_t resident_groups(const ResidentPlan &p, int device) {
   return (uint32_t)std::max(n, 0);
 }
 
-// Microseconds of a step of one wave of groups, fitted to slopes over 200 to
-// 2000 moments on square, Rashba and honeycomb lattices of 128 to 32k rows:
-// a fixed part (for a cluster more than half of it the barrier's release and
-// a distributed-shared-memory round trip) and the entries of a block, which
-// cost shared-memory wavefronts unless they live in registers.  Measured for
-// FP64 real / complex, one source: 0.43 / 0.67 us at 512 rows, 0.56 / 0.71 at
-// 1800, 0.65 / 0.85 at 8192; doubling steps 0.61 / 0.71 / 0.79; a batch of 128
-// sources of 1800 rows 1.7 / 3.6.
-static double wave_us(const ResidentPlan &p) {
-  static const double block0[4] = {0.42, 0.30, 0.45, 0.32}, reg0[4] = {0.68, 0.56, 0.72, 0.58};
-  static const double smem_ns[4] = {0.22, 0.14, 0.18, 0.15}, reg_ns[4] = {0.07, 0.04, 0.08, 0.045};
-  const double fixed = (p.cluster == 1 ? block0[p.kind] : p.reg ? reg0[p.kind] : 0.45) + (p.dots ? 0.17 : 0.0);
-  const double per_entry = (p.reg ? reg_ns : smem_ns)[p.kind] * 1e-3 *
-                           (p.cols == 1 ? 1.0 : p.cols == 2 ? 1.15 : 1.5);
-  return fixed + 32.0 * p.chunks * per_entry;
+// Microseconds of a step of `waves` waves of groups, fitted (1400 batches of 1 to
+// 128 sources on square, Rashba, honeycomb and cubic lattices of 50 to 80k rows,
+// all shapes) to nine in ten times within 13%, all within a third.  A fixed
+// part (for a cluster more than half of it the barrier's release and a
+// distributed-shared-memory round trip), the entries of a block, which cost
+// shared-memory wavefronts unless they live in registers, more where several
+// blocks share an SM, and the doubling sums.  Measured for FP64 real / complex,
+// one source: 0.65 / 0.83 us at 512 rows, 0.74 / 0.93 at 1800, 0.80 / 1.2 at
+// 8192; a batch of 128 sources of 1800 rows 2.1 / 4.3.
+static double wave_us(const ResidentPlan &p, uint32_t groups_at_once, uint32_t sms) {
+  static const double base[2][4] = {{0.74, 0.45, 0.45, 0.52}, {0.49, 0.34, 0.64, 0.35}};
+  static const double entry_ns[2][4] = {{0.168, 0.129, 0.205, 0.135}, {0.122, 0.044, 0.073, 0.044}};
+  static const double wider[2][2] = {{1.26, 1.88}, {1.87, 3.78}};  // two and four columns
+  static const double column[4] = {0.0, 0.09, 0.22, 0.086};
+  const int reg = p.reg ? 1 : 0;
+  const double blocks = std::min(std::ceil((double)p.groups * p.cluster / sms),
+                                 (double)groups_at_once * p.cluster / sms);
+  const double per_entry = entry_ns[reg][p.kind] * (p.cols == 1 ? 1.0 : wider[reg][p.cols == 4]) +
+                           0.1 * std::max(blocks - 1, 0.0);
+  double us = base[reg][p.kind] + (p.cluster > 1 ? 0.295 : 0.0) + 32e-3 * p.chunks * per_entry +
+              column[p.kind] * (p.cols - 1);
+  if (p.dots) us += 0.18 * (1 + 0.4 * (p.cols - 1));
+  if (p.cap == 0) us += 1.2;  // moments stored step by step
+  return us * ((p.groups + groups_at_once - 1) / groups_at_once);
 }
 
-// The same for a step of the launched kernels: launch latency, dependent
-// round trips and the fewest bytes at 5 TB/s (us measured at 2k-64k rows: 4.1
-// to 5.1 for one source, 6.2 to 10 for a batch; the doubling step is two
-// launches, 10.3 to 37).
+// The same for a dependent step of the launched kernels, by padded width:
+// launch, round trips, rows and entries of the columns.  Nine in ten times
+// within 14%, all within a third.  Measured at 1800 / 16k / 51k rows: FP64
+// real, one source 3.2 / 3.2 / 2.6 us, 16 sources 3.9 / 4.4 / 5.9, 128 4.3 /
+// 10.8 / 29; doubling steps, real, 1 source 2.9 / 2.9 / 3.1, 16 4.4 / 5.3 / 6.7,
+// 128 6.5 / 11.8 / 23.
 static double launch_us(const tbtkkpm_matrix *m, int kind, bool dots, uint32_t B) {
-  const double bytes = 32.0 * m->chunks * (value_size(kind) + 4) + 3.0 * m->N * B * vec_elem_size(kind);
-  return (B == 1 ? 4.0 : 5.5) + (dots ? 3.0 : 0.0) + bytes / 5e6;
+  struct Fit { double fixed, doubling, row, entry; };  // us, us per doubled width, ps per row and entry
+  static const Fit direct[4] = {{2.7, 0.22, 2.3, 0.94}, {2.65, 0.25, 1.1, 0.45}, {2.81, 0.28, 0, 0.78}, {2.39, 0.26, 0.09, 0.42}};
+  static const Fit doubled[2] = {{3.06, 0.38, 0, 0.87}, {2.73, 0.41, 0.74, 0.41}};
+  const Fit &f = dots ? doubled[kind - kVecC64] : direct[kind];
+  int log2w = 0;
+  while ((1u << log2w) < B) log2w++;
+  return f.fixed + f.doubling * log2w +
+         1e-6 * (double)(1u << log2w) * (f.row * m->N + f.entry * 32.0 * m->chunks);
 }
 
 int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint32_t *trow,
@@ -152,8 +172,13 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
     if (e != cudaSuccess) return cuda_fail(e, "recursion: slice bounds");
     m->host_slice_ptr = std::move(sp);
   }
-  // a tenth below the launched step, for the error of both estimates
-  double best = 0.9 * launch_us(m, kind, dots, B);
+  // Below the launched step by a margin for the error of both estimates.  Over
+  // those 1400 batches the rule's choice is within 5% of the launched step or
+  // faster but for four (at most 1.16), and 0.6% from the best shape on average;
+  // estimates of the steps before they were dependent launches sent batches on
+  // chip that were up to 1.5 times faster launched (16k to 50k rows, 2-128
+  // sources).
+  double best = 0.95 * launch_us(m, kind, dots, B);
   for (uint32_t C = 1; C <= kResMaxCluster; C *= 2)
     for (uint32_t cols = 1; cols <= std::min(max_cols(kind), 2 * B - 1); cols *= 2) {
       ResidentPlan p{};
@@ -163,7 +188,7 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
       p.cols = cols;
       p.groups = (B + cols - 1) / cols;
       if (!shape_resident(m, trow, tcol, T, p)) continue;
-      if (wave_us(p) >= best) continue;
+      if (wave_us(p, p.groups, p.groups * p.cluster) >= best) continue;  // at least that
       const uint64_t key = ((((uint64_t)kind * 2 + dots) * 32 + C) * 8 + cols) << 32 | p.smem;
       auto it = m->resident_groups.find(key);
       if (it == m->resident_groups.end()) {
@@ -171,8 +196,7 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
         it = m->resident_groups.emplace(key, resident_groups(p, m->device)).first;
       }
       if (it->second == 0) continue;
-      const uint32_t waves = (p.groups + it->second - 1) / it->second;
-      const double us = wave_us(p) * (waves == 1 ? 1.0 : 1.1 * waves);
+      const double us = wave_us(p, it->second, (uint32_t)sm_count(m->device));
       if (us >= best) continue;
       best = us;
       p.ok = true;
