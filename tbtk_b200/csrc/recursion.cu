@@ -1346,13 +1346,14 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   const bool real64 = ldos && real64_mode(m, precision);
   const StepEntry *best = nullptr, *best_cplx = nullptr;
   double best_ms = 0, best_cplx_ms = 0;
-  // best of two runs of a step kernel (null: the untuned default) in ms per
-  // step, or -1 for a tile-staged step whose ring does not fit this matrix
-  auto time_step = [&](const StepEntry *e, double &ms) -> int {
+  // best of two runs of a step kernel (null: the untuned default, on vectors of
+  // doubles if `r64`) in ms per step, or -1 for a tile-staged step whose ring
+  // does not fit this matrix
+  auto time_step = [&](const StepEntry *e, bool r64, double &ms) -> int {
     for (int rep = 0; rep < 2; rep++) {
       m->timer.recursion_ms = 0;
       RunOptions opt;
-      opt.use_real64 = real64;
+      opt.use_real64 = r64;
       opt.head = false;
       opt.force = e;
       opt.untuned = true;
@@ -1375,7 +1376,7 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
     if ((uint32_t)(t[i].tpr * t[i].vpt) != Bp) continue;
     if (t[i].cls == kClassFP64Real && !real64) continue;
     double ms = 0;
-    if ((rc = time_step(&t[i], ms))) break;
+    if ((rc = time_step(&t[i], real64, ms))) break;
     if (ms < 0) continue;
     if (!best || ms < best_ms) {
       best = &t[i];
@@ -1387,16 +1388,23 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
     }
   }
   // The default of a batch that runs on chip stays where it beats every step
-  // kernel: no configuration is recorded then.
-  bool keep_default = false;
-  ResidentPlan res;
-  const int kind = real ? kVecF32 : is_mixed(precision) ? kVecC64 : real64 ? kVecF64R : kVecF64C;
-  if (!rc) rc = plan_resident(m, kind, doubling, B, tl.row.data(), tl.col.data(), B, res);
-  if (!rc && res.ok) {
+  // kernel: no configuration is recorded then.  Complex vectors, which the
+  // moment calls of a real matrix take, are compared by themselves.
+  auto default_wins = [&](int kind, const StepEntry *e, double step_ms, bool &wins) -> int {
+    wins = false;
+    if (!e) return TBTKKPM_OK;
+    ResidentPlan res;
+    int r = plan_resident(m, kind, doubling, B, tl.row.data(), tl.col.data(), B, res);
+    if (r || !res.ok) return r;
     double ms = 0;
-    rc = time_step(nullptr, ms);
-    keep_default = !rc && best && ms < best_ms;
-  }
+    if ((r = time_step(nullptr, kind == kVecF64R, ms))) return r;
+    wins = ms < step_ms;
+    return TBTKKPM_OK;
+  };
+  const int kind = real ? kVecF32 : is_mixed(precision) ? kVecC64 : real64 ? kVecF64R : kVecF64C;
+  bool keep_default = false, keep_cplx = false;
+  if (!rc) rc = default_wins(kind, best, best_ms, keep_default);
+  if (!rc && real64) rc = default_wins(kVecF64C, best_cplx, best_cplx_ms, keep_cplx);
   const bool created = saved.ev[0] == nullptr;
   if (created) m->timer.destroy();
   else {
@@ -1408,10 +1416,10 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   }
   if (rc) return rc;
   if (!best) return fail(TBTKKPM_ERR_UNSUPPORTED, "matrix_autotune: no configuration for %u", B);
-  auto keep = [&](int key, const StepEntry *e) {
+  auto keep = [&](int key, const StepEntry *e, bool untuned) {
     if (!e) return;
     std::lock_guard<std::mutex> lk(g_tuned_mu);
-    if (keep_default) {
+    if (untuned) {
       m->tuned.erase(tune_key(key, Bp));
       g_tuned.erase(shape_key(m, key, Bp));
       return;
@@ -1419,8 +1427,12 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
     m->tuned[tune_key(key, Bp)] = {e->tpr, e->vpt, e->minb};
     g_tuned[shape_key(m, key, Bp)] = {e->tpr, e->vpt, e->minb};
   };
-  if (real64) keep(kClassFP64Real, best);
-  keep(cls, real64 ? best_cplx : best);
+  if (real64) {
+    keep(kClassFP64Real, best, keep_default);
+    keep(cls, best_cplx, keep_cplx);
+  } else {
+    keep(cls, best, keep_default);
+  }
   if (tpr) *tpr = best->tpr;
   if (vpt) *vpt = best->vpt;
   if (minb) *minb = best->minb;
