@@ -257,10 +257,12 @@ TBTKKPM_API int tbtkkpm_ldos(
  * on this handle.  ldos != 0 tunes the kernels tbtkkpm_ldos_sites uses (the
  * dot-product variant at TBTKKPM_MIXED), 0 those of the moment calls.
  * A small matrix whose recursion runs on chip by default keeps that when it is
- * faster than every configuration; the outputs are the fastest
- * configuration's all the same.
+ * faster than every configuration; the outputs then are (1, padded width, 0),
+ * the default of the width.
  * Outputs (may be NULL): the chosen configuration and its ms per step.
- * tbtkkpm_matrix_set_config installs a known choice without timing.
+ * tbtkkpm_matrix_set_config installs a known choice without timing.  Any but
+ * (1, width, 0) makes batches of that width launched steps of that
+ * configuration, also where they would run on chip.
  * (No reference counterpart.) */
 TBTKKPM_API int tbtkkpm_matrix_autotune(
 	tbtkkpm_matrix *m, uint32_t B, int precision, int ldos,
@@ -278,7 +280,9 @@ TBTKKPM_API int tbtkkpm_matrix_set_config(
  * kernels (real matrices at the mixed precisions): cap + 100*8 (802, 803)
  * keeps the doubling dot sums in shared memory instead of registers;
  * 100000 + 1000000*CV + 1000*R + 10*CW + BPS a tile-staged step of R-row
- * tiles (CV 200: FP64 on vectors of doubles, for a real matrix's sums).
+ * tiles (CV 200: FP64 on vectors of doubles, for a real matrix's sums);
+ * (1, width, 0), listed for every width, is the default, chosen by the matrix
+ * and on chip for a small one.
  * (No reference counterpart.) */
 TBTKKPM_API int tbtkkpm_step_configs(int precision, int ldos, int *out, int cap);
 

@@ -241,9 +241,12 @@ ShapeKey shape_key(const tbtkkpm_matrix *m, int cls, uint32_t Bp) {
   return {(uint64_t)m->device, (uint64_t)cls, Bp, m->N, m->nnz};
 }
 
+// The configuration (1, padded width, kUntuned): none, the default of the width.
+constexpr int kUntuned = 0;
+
 // The configuration chosen for a batch by set_config or the autotuner: the
 // handle's for this (class, padded width), else this process's for a matrix
-// of the same shape; null where none was.
+// of the same shape; null where none was, or where the default was chosen.
 const StepEntry *tuned_step(const tbtkkpm_matrix *m, int precision, bool dots, uint32_t B,
                             bool real64) {
   const bool real = real_mode(m, precision);
@@ -251,6 +254,7 @@ const StepEntry *tuned_step(const tbtkkpm_matrix *m, int precision, bool dots, u
   const uint32_t Bp = shape_for(precision, B, real, dots, m->N).bp();
   auto it = m->tuned.find(tune_key(key, Bp));
   if (it != m->tuned.end()) {
+    if (it->second[2] == kUntuned) return nullptr;
     const StepEntry *e = find_step(cls, it->second[0], it->second[1], it->second[2]);
     if (e) return e;
   }
@@ -1309,7 +1313,8 @@ int tbtkkpm::ldos_sites_terms(tbtkkpm_matrix *m, tbtkkpm_table *t, uint32_t M, c
 // sources on this matrix (probe_steps steps each, best of two runs, CUDA
 // events on the handle's stream around the steps) and keeps the fastest for
 // later batches of that width on this handle, unless such batches run on
-// chip and that is faster still.
+// chip and that is faster still: then none is kept, and the outputs say so
+// (kUntuned), so that a saved result brings the same default back.
 extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precision, int ldos,
                                        uint32_t probe_steps, int *tpr, int *vpt, int *minb,
                                        double *ms_per_step) {
@@ -1390,15 +1395,15 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   // The default of a batch that runs on chip stays where it beats every step
   // kernel: no configuration is recorded then.  Complex vectors, which the
   // moment calls of a real matrix take, are compared by themselves.
-  auto default_wins = [&](int kind, const StepEntry *e, double step_ms, bool &wins) -> int {
+  auto default_wins = [&](int kind, const StepEntry *e, double &ms, bool &wins) -> int {
     wins = false;
     if (!e) return TBTKKPM_OK;
     ResidentPlan res;
     int r = plan_resident(m, kind, doubling, B, tl.row.data(), tl.col.data(), B, res);
     if (r || !res.ok) return r;
-    double ms = 0;
-    if ((r = time_step(nullptr, kind == kVecF64R, ms))) return r;
-    wins = ms < step_ms;
+    double chip_ms = 0;
+    if ((r = time_step(nullptr, kind == kVecF64R, chip_ms))) return r;
+    if ((wins = chip_ms < ms)) ms = chip_ms;
     return TBTKKPM_OK;
   };
   const int kind = real ? kVecF32 : is_mixed(precision) ? kVecC64 : real64 ? kVecF64R : kVecF64C;
@@ -1433,15 +1438,15 @@ extern "C" int tbtkkpm_matrix_autotune(tbtkkpm_matrix *m, uint32_t B, int precis
   } else {
     keep(cls, best, keep_default);
   }
-  if (tpr) *tpr = best->tpr;
-  if (vpt) *vpt = best->vpt;
-  if (minb) *minb = best->minb;
+  if (tpr) *tpr = keep_default ? 1 : best->tpr;
+  if (vpt) *vpt = keep_default ? (int)Bp : best->vpt;
+  if (minb) *minb = keep_default ? kUntuned : best->minb;
   if (ms_per_step) *ms_per_step = best_ms;
   return TBTKKPM_OK;
 }
 
 // Records a configuration for batches of B sources without timing (a
-// cached autotuner result).
+// cached autotuner result); kUntuned: the default, whatever else was chosen.
 extern "C" int tbtkkpm_matrix_set_config(tbtkkpm_matrix *m, uint32_t B, int precision, int ldos,
                                          int tpr, int vpt, int minb) {
   int rc = check_precision(precision);
@@ -1451,7 +1456,8 @@ extern "C" int tbtkkpm_matrix_set_config(tbtkkpm_matrix *m, uint32_t B, int prec
   const bool real = real_mode(m, precision);
   const int cls = step_class(precision, doubling, real);
   const uint32_t Bp = shape_for(precision, std::max(B, 1u), real).bp();
-  if ((uint32_t)(tpr * vpt) != Bp || !find_step(cls, tpr, vpt, minb))
+  const bool untuned = tpr == 1 && minb == kUntuned;
+  if ((uint32_t)(tpr * vpt) != Bp || (!untuned && !find_step(cls, tpr, vpt, minb)))
     return fail(TBTKKPM_ERR_ARGUMENT, "matrix_set_config: no compiled configuration %d x %d / %d "
                 "for %u columns", tpr, vpt, minb, Bp);
   std::lock_guard<std::mutex> lk(m->lock);
@@ -1460,20 +1466,30 @@ extern "C" int tbtkkpm_matrix_set_config(tbtkkpm_matrix *m, uint32_t B, int prec
   return TBTKKPM_OK;
 }
 
-// The compiled step configurations of the kernel class a call at this
-// precision uses (ldos != 0: tbtkkpm_ldos_sites), as (tpr, vpt, variant)
-// triples; returns how many there are (writes at most cap triples).
-extern "C" int tbtkkpm_step_configs(int precision, int ldos, int *out, int cap) {
-  if (check_precision(precision)) return -1;
+// Lists a class's step configurations, and the default of each of its widths,
+// as (tpr, vpt, variant) triples; returns how many there are (writes at most
+// cap triples).
+static int list_configs(int cls, int *out, int cap) {
   const StepEntry *t;
   int n;
-  step_table(step_class(precision, ldos && precision == TBTKKPM_MIXED), &t, &n);
-  for (int i = 0; i < n && i < cap && out; i++) {
-    out[3 * i] = t[i].tpr;
-    out[3 * i + 1] = t[i].vpt;
-    out[3 * i + 2] = t[i].minb;
+  step_table(cls, &t, &n);
+  std::vector<std::array<int, 3>> all;
+  std::vector<int> widths;
+  for (int i = 0; i < n; i++) {
+    all.push_back({t[i].tpr, t[i].vpt, t[i].minb});
+    const int w = t[i].tpr * t[i].vpt;
+    if (std::find(widths.begin(), widths.end(), w) == widths.end()) widths.push_back(w);
   }
-  return n;
+  for (int w : widths) all.push_back({1, w, kUntuned});
+  for (int i = 0; i < (int)all.size() && i < cap && out; i++) std::copy(all[i].begin(), all[i].end(), out + 3 * i);
+  return (int)all.size();
+}
+
+// The step configurations of the kernel class a call at this precision uses
+// (ldos != 0: tbtkkpm_ldos_sites).
+extern "C" int tbtkkpm_step_configs(int precision, int ldos, int *out, int cap) {
+  if (check_precision(precision)) return -1;
+  return list_configs(step_class(precision, ldos && precision == TBTKKPM_MIXED), out, cap);
 }
 
 // As tbtkkpm_step_configs for the kernels this matrix uses (real-vector
@@ -1481,16 +1497,8 @@ extern "C" int tbtkkpm_step_configs(int precision, int ldos, int *out, int cap) 
 extern "C" int tbtkkpm_matrix_step_configs(tbtkkpm_matrix *m, int precision, int ldos, int *out,
                                            int cap) {
   if (!m || check_precision(precision)) return -1;
-  const StepEntry *t;
-  int n;
-  step_table(step_class(precision, ldos && precision == TBTKKPM_MIXED, real_mode(m, precision)),
-             &t, &n);
-  for (int i = 0; i < n && i < cap && out; i++) {
-    out[3 * i] = t[i].tpr;
-    out[3 * i + 1] = t[i].vpt;
-    out[3 * i + 2] = t[i].minb;
-  }
-  return n;
+  return list_configs(step_class(precision, ldos && precision == TBTKKPM_MIXED, real_mode(m, precision)),
+                      out, cap);
 }
 
 extern "C" int tbtkkpm_matrix_set_real(tbtkkpm_matrix *m, int enable) {

@@ -132,7 +132,8 @@ STAT_NAMES = ["completed", "p50_ms", "p99_ms", "mean_ms", "reruns", "ticks", "st
 def step_configs(precision, ldos=True):
     """Compiled step configurations (tpr, vpt, variant) of the kernels a call
     at this precision uses; variant 2-4 is a register cap, 100 + 10*S + W a
-    bulk-copy kernel with S stages per warp and W warps per block."""
+    bulk-copy kernel with S stages per warp and W warps per block; (1, width,
+    0) is the default of a width."""
     lib = load_library()
     n = lib.tbtkkpm_step_configs(int(precision), int(bool(ldos)), None, 0)
     if n < 0:
@@ -268,7 +269,8 @@ class Matrix:
     def autotune(self, B, precision, ldos=True, probe_steps=8):
         """Times the compiled step configurations for batches of B sources
         and keeps the fastest on this handle; returns (tpr, vpt, minb,
-        ms per step)."""
+        ms per step), (1, width, 0, ms) where the default, on chip, is faster
+        than all of them.  set_config takes either back."""
         t = ctypes.c_int()
         v = ctypes.c_int()
         mb = ctypes.c_int()

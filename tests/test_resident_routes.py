@@ -66,3 +66,29 @@ def test_tuning_sums_keeps_moments_on_chip(gpu, side):
     sites = np.arange(4, dtype=np.uint32)
     assert _ldos_launches(gpu, m, sites, gpu.FP64) < 20
     assert _launches(gpu, lambda: m.moments_batched(sites, sites, sites, M, 1e-3, gpu.FP64)) < 20
+
+
+@pytest.mark.parametrize("precision", ["FP64", "MIXED"])
+@pytest.mark.parametrize("alpha", [0.0, 0.3])
+def test_saved_tuning_result_keeps_the_chip(gpu, alpha, precision):
+    """What the autotuner returns for a small matrix, installed on a new
+    handle, leaves its calls where tuning left them; another configuration
+    makes them launched steps, until the default is installed again."""
+    csr = L.square(30, 30, t=1.0, J=0.5, W=2.0, alpha=alpha, periodic=True, seed=3).csr()
+    p, sites = getattr(gpu, precision), np.arange(4, dtype=np.uint32)
+    m = gpu.Matrix.from_csr(*csr, SCALE)
+    tuned = m.autotune(4, p, ldos=True, probe_steps=64)
+    assert tuned[:3] in m.configs_for(4, p, True) and tuned[3] > 0
+    assert _ldos_launches(gpu, m, sites, p) < 20
+    fresh = gpu.Matrix.from_csr(*csr, SCALE)
+    fresh.set_fp64_head(0)
+    fresh.set_config(4, p, *tuned[:3], ldos=True)
+    assert _ldos_launches(gpu, fresh, sites, p) < 20
+    other = [c for c in fresh.configs_for(4, p, True) if 1 <= c[2] <= 4][0]
+    fresh.set_config(4, p, *other, ldos=True)
+    assert _ldos_launches(gpu, fresh, sites, p) >= M // 2
+    fresh.set_config(4, p, 1, 4, 0, ldos=True)
+    assert _ldos_launches(gpu, fresh, sites, p) < 20
+    for bad in ((1, 8, 0), (2, 2, 0), (4, 1, 0)):
+        with pytest.raises(gpu.TBTKError):
+            fresh.set_config(4, p, *bad, ldos=True)
