@@ -119,8 +119,7 @@ struct Model {
   uint32_t tcount = 0;
   bool dirty = true;
   DevBuf lane_mem;  // one allocation; the lane buffers above are views into it
-  // gather plans of the matrix by 2 * rows per tile + complex, 1024 more for
-  // rows of at most 32 bytes (null: none)
+  // gather plans of the matrix by model_plan's key (null: none)
   std::map<int, const TilePlan *> plans;
   void release_lanes() {
     for (DevBuf *b : {&vec[0], &vec[1], &dots, &mu, &mu_direct, &base, &laneM, &bitmap, &tlist,
@@ -182,12 +181,16 @@ const MultiEntry *find_multi(int tpr, int vpt, int minb, bool real) {
 // Gather plan of a model for a tile-staged entry (built on first use on the
 // model's matrix handle); null when the entry is register-staged, rows of W
 // lanes are too narrow for bulk copies, or the matrix has a tile the plan
-// builder cannot take.
-const TilePlan *model_plan(Model *m, uint32_t W, const MultiEntry *e, int *rc) {
+// builder cannot take.  few_copies: columns are staged four at a time where
+// that makes far fewer copies (a honeycomb's runs of two rows), as in
+// fitting_plan of recursion.cu; such copies may run three rows past a vector's
+// end (make_resident).
+const TilePlan *model_plan(Model *m, uint32_t W, const MultiEntry *e, bool few_copies, int *rc) {
   *rc = TBTKKPM_OK;
   if (!is_multi_tiled(e->minb) || (W * m->esize()) % 16 != 0) return nullptr;
   const bool narrow = W * m->esize() <= 32;
-  const int R = multi_tiled_rows(e->minb), key = (narrow ? 1024 : 0) + 2 * R + (m->real ? 0 : 1);
+  const int R = multi_tiled_rows(e->minb);
+  const int key = (few_copies ? narrow ? 2048 : 1024 : 0) + 2 * R + (m->real ? 0 : 1);
   auto it = m->plans.find(key);
   if (it != m->plans.end()) return it->second;
   // the first use builds it on the matrix handle (under its lock: the rerun
@@ -196,10 +199,7 @@ const TilePlan *model_plan(Model *m, uint32_t W, const MultiEntry *e, int *rc) {
   {
     std::lock_guard<std::mutex> lk(m->mat->lock);
     *rc = tile_plan(m->mat, R, !m->real, &p);
-    // Columns four at a time where that makes far fewer copies (a honeycomb's
-    // runs of two rows), as in fitting_plan of recursion.cu.  The copies may
-    // run three rows past a vector's end (make_resident).
-    if (!*rc && p && (narrow || p->nruns > (uint64_t)p->ntiles * (4 + R / 16))) {
+    if (few_copies && !*rc && p && (narrow || p->nruns > (uint64_t)p->ntiles * (4 + R / 16))) {
       const TilePlan *four = nullptr;
       *rc = tile_plan(m->mat, R, !m->real, &four, false, 4);
       if (!*rc && four && 2 * (uint64_t)four->nruns <= p->nruns) p = four;
@@ -222,6 +222,29 @@ TiledLayout multi_layout(const MultiEntry *e, uint32_t W, bool real, uint32_t wm
   return tiled_layout(p, W * (uint32_t)(real ? sizeof(float) : sizeof(float2)),
                       real ? (uint32_t)sizeof(double) : (uint32_t)sizeof(double2),
                       tiled_budget(multi_tiled_bps(e->minb)) - (kMultiHeader - kTiledHeader));
+}
+
+// The plans tp of the models of a class (lanes W wide, real or complex) for a
+// tile-staged entry and the ring `ly` they share; false where a model has no
+// plan or no ring of two stages fits.  Columns staged four at a time take more
+// room; where they leave none, every model stages them one at a time.
+bool class_plans(const std::vector<Model *> &models, uint32_t W, const MultiEntry *e, bool real,
+                 std::vector<const TilePlan *> &tp, TiledLayout &ly, int *rc) {
+  *rc = TBTKKPM_OK;
+  for (const bool few_copies : {true, false}) {
+    uint32_t wmax = 0, umax = 0;
+    tp.clear();
+    for (Model *m : models) {
+      const TilePlan *p = model_plan(m, W, e, few_copies, rc);
+      if (*rc || !p) return false;
+      tp.push_back(p);
+      wmax = std::max(wmax, p->wmax);
+      umax = std::max(umax, p->umax);
+    }
+    ly = multi_layout(e, W, real, wmax, umax);
+    if (ly.stages) return true;
+  }
+  return false;
 }
 
 // Register-staged shape per width and class (few threads per row, several
@@ -719,23 +742,13 @@ int plan_tick(tbtkkpm_server *s, std::vector<ClassPlan> &plans) {
     ClassPlan &cp = plans[c];
     std::vector<const TilePlan *> tp(members[c].size(), nullptr);
     if (is_multi_tiled(cp.entry->minb)) {
-      uint32_t wmax = 0, umax = 0;
-      bool ok = true;
-      for (size_t i = 0; i < members[c].size() && ok; i++) {
-        int rc;
-        tp[i] = model_plan(members[c][i], cp.W, cp.entry, &rc);
-        if (rc) return rc;
-        ok = tp[i] != nullptr;
-        if (ok) {
-          wmax = std::max(wmax, tp[i]->wmax);
-          umax = std::max(umax, tp[i]->umax);
-        }
-      }
-      if (ok) cp.ly = multi_layout(cp.entry, cp.W, cp.real, wmax, umax);
-      if (!ok || cp.ly.stages == 0) {
+      int rc;
+      const bool fits = class_plans(members[c], cp.W, cp.entry, cp.real, tp, cp.ly, &rc);
+      if (rc) return rc;
+      if (!fits) {
         const auto d = register_config(cp.W, cp.real);
         cp.entry = find_multi(d[0], d[1], d[2], cp.real);
-        std::fill(tp.begin(), tp.end(), nullptr);
+        tp.assign(members[c].size(), nullptr);
       }
     }
     for (size_t i = 0; i < members[c].size(); i++) {
@@ -1874,13 +1887,14 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
     const MultiEntry &en = *ep;
     if ((uint32_t)(en.tpr * en.vpt) != W) continue;
     // a tile-staged entry needs the probe's plan and a ring that fits
-    const TilePlan *plan = model_plan(probe, W, &en, &rc);
-    if (rc) break;
+    const TilePlan *plan = nullptr;
     TiledLayout ly{};
     if (is_multi_tiled(en.minb)) {
-      if (!plan) continue;
-      ly = multi_layout(&en, W, real, plan->wmax, plan->umax);
-      if (ly.stages == 0) continue;
+      std::vector<const TilePlan *> tp;
+      const bool fits = class_plans({probe}, W, &en, real, tp, ly, &rc);
+      if (rc) break;
+      if (!fits) continue;
+      plan = tp[0];
     }
     MultiModel d{};
     d.A.slice_ptr = probe->mat->slice_ptr.as<uint32_t>();
@@ -1978,7 +1992,10 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
   // the first tick that needs them
   for (auto &p : s->models) {
     if (p->Wmax < W || (!s->adaptive_width && p->Wmax != W) || p->real != real) continue;
-    model_plan(p.get(), W, best, &rc);
+    if (!is_multi_tiled(best->minb)) break;
+    std::vector<const TilePlan *> tp;
+    TiledLayout ly;
+    class_plans({p.get()}, W, best, real, tp, ly, &rc);
     if (rc) return rc;
   }
   *best_out = best;
