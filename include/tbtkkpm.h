@@ -431,7 +431,10 @@ TBTKKPM_API int tbtkkpm_expectation_values(
  * bits alone or among any other requests.  Lane memory (vectors, moments)
  * of a model is allocated when it first gets a request and counts against
  * `hbm_budget` (bytes); idle models are evicted least recently used first;
- * a request whose model does not fit waits.  Any thread may submit and
+ * a request whose model does not fit waits.  Outside the budget lie the
+ * matrices, the tables and the scratch of the FP64 head: 0.06 MB (real) or
+ * 0.11 MB (complex) an entry of the widest row, up to 10, and 0.3 MB more for a
+ * complex model, for each lane that starts, of at most one per SM at once.  Any thread may submit and
  * wait; one worker thread per server drives the device. */
 
 typedef struct tbtkkpm_server tbtkkpm_server;

@@ -41,7 +41,6 @@ constexpr uint32_t kPrefixRows = 6144;     // rows of one source's ball
 constexpr uint32_t kPrefixSlots = 8192;    // hash slots (power of two, above the rows)
 constexpr uint32_t kPrefixSlotBits = 13;
 constexpr uint32_t kPrefixEmpty = 0xffffffffu;
-constexpr uint32_t kPrefixMaxJobs = 256;   // sources of one launch
 constexpr int kPrefixBlock = 1024;
 constexpr int kPrefixWidth = 10;           // most entries of a row kept in scratch
 constexpr uint16_t kPrefixNone = 0xffffu;  // an entry whose column is not in the ball
@@ -52,10 +51,12 @@ constexpr double kPrefixUnit = 1.0 / 2305843009213693952.0;   // 2^-61
 // rotation)
 constexpr size_t kPrefixTable = (size_t)kPrefixSlots * 4 + (size_t)kPrefixRows * 4 + (size_t)kPrefixSlots * 2;
 __host__ __device__ constexpr size_t prefix_smem(bool real) { return kPrefixTable + (real ? 3 * (size_t)kPrefixRows * 8 : 0); }
-// global scratch of a source: values [width][rows], complex vectors
-// v[3][rows], local indices [width][rows] u16
-__host__ __device__ constexpr size_t prefix_scratch(bool real) {
-  return (size_t)kPrefixWidth * kPrefixRows * ((real ? 8 : 16) + 2) + (real ? 0 : 3 * (size_t)kPrefixRows * 16);
+// global scratch of a source: values [lists][rows], complex vectors
+// v[3][rows], local indices [lists][rows] u16, with `lists` the widest slice of
+// up to kPrefixWidth entries among the sources' matrices: 0.31 MB on a square
+// lattice, 1.29 on a Rashba one
+__host__ __device__ constexpr size_t prefix_scratch(bool real, uint32_t lists) {
+  return (size_t)lists * kPrefixRows * ((real ? 8 : 16) + 2) + (real ? 0 : 3 * (size_t)kPrefixRows * 16);
 }
 
 struct PrefixJob {
@@ -141,7 +142,7 @@ __device__ __forceinline__ uint32_t prefix_enter(uint32_t *key, uint32_t row) {
 // elsewhere beforehand), rounded once to FP32.
 template <bool REAL>
 __global__ void __launch_bounds__(kPrefixBlock, 1)
-kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, PrefixResult *res) {
+kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, uint32_t lists, PrefixResult *res) {
   using V = PrefixVec<REAL>;
   using T = typename V::T;
   constexpr int L = 5;  // entries loaded together
@@ -152,12 +153,12 @@ kpm_prefix(const PrefixJob *__restrict__ jobs, char *scratch, PrefixResult *res)
   uint32_t *key = reinterpret_cast<uint32_t *>(prefix_mem);
   uint32_t *rows = key + kPrefixSlots;
   uint16_t *index = reinterpret_cast<uint16_t *>(rows + kPrefixRows);
-  char *mine = scratch + (size_t)blockIdx.x * prefix_scratch(REAL);
+  char *mine = scratch + (size_t)blockIdx.x * prefix_scratch(REAL, lists);
   T *val = reinterpret_cast<T *>(mine);
-  T *v = REAL ? reinterpret_cast<T *>(index + kPrefixSlots) : val + (size_t)kPrefixWidth * kPrefixRows;
-  uint16_t *nbr = reinterpret_cast<uint16_t *>(val + (size_t)(kPrefixWidth + (REAL ? 0 : 3)) * kPrefixRows);
+  T *v = REAL ? reinterpret_cast<T *>(index + kPrefixSlots) : val + (size_t)lists * kPrefixRows;
+  uint16_t *nbr = reinterpret_cast<uint16_t *>(val + (size_t)(lists + (REAL ? 0 : 3)) * kPrefixRows);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool listed = J.width <= (uint32_t)kPrefixWidth;
+  const bool listed = J.width <= lists;
   for (uint32_t i = threadIdx.x; i < kPrefixSlots; i += kPrefixBlock) key[i] = kPrefixEmpty;
   if (threadIdx.x == 0) {
     s_count = 0;
@@ -380,12 +381,13 @@ static __global__ void k_pattern_check(uint32_t N, const uint32_t *__restrict__ 
 
 namespace tbtkkpm {
 
-// Runs the FP64 head of `jobs` on stream st, kPrefixMaxJobs sources per
-// launch (the scratch is reused), those with real buffers apart from the
-// others; every source with q >= 2 leaves j_q and j_{q-1} in its buffers.
-// res[i] receives the steps source i reached and its rows.  Returns after the
-// stream has passed the last launch.
-static int run_fp64_head(cudaStream_t st, const std::vector<PrefixJob> &jobs, Workspace &ws,
+// Runs the FP64 head of `jobs` on stream st, those with real buffers apart from
+// the others; every source with q >= 2 leaves j_q and j_{q-1} in its buffers.
+// res[i] receives the steps source i reached and its rows.  A launch takes as
+// many sources as run at once, a block per SM, and the next one reuses their
+// scratch; fewer when that cannot be allocated.  Returns after the stream has
+// passed the last launch.
+static int run_fp64_head(cudaStream_t st, int device, const std::vector<PrefixJob> &jobs, Workspace &ws,
                          std::vector<PrefixResult> &res) {
   const size_t nj = jobs.size();
   res.assign(nj, PrefixResult{0, 0});
@@ -397,13 +399,24 @@ static int run_fp64_head(cudaStream_t st, const std::vector<PrefixJob> &jobs, Wo
   for (size_t i = 0, k = nreal; i < nj; i++)
     if (!jobs[i].real) order[k++] = (uint32_t)i;
   std::vector<PrefixJob> sorted(nj);
-  for (size_t i = 0; i < nj; i++) sorted[i] = jobs[order[i]];
-  const size_t most_real = std::min<size_t>(nreal, kPrefixMaxJobs), most = std::min<size_t>(nj - nreal, kPrefixMaxJobs);
+  uint32_t lists[2] = {0, 0};  // complex, real
+  for (size_t i = 0; i < nj; i++) {
+    sorted[i] = jobs[order[i]];
+    uint32_t &l = lists[i < nreal];
+    if (sorted[i].width <= (uint32_t)kPrefixWidth) l = std::max(l, sorted[i].width);
+  }
   int rc;
-  if ((rc = ws.head.reserve(std::max(prefix_scratch(true) * most_real, prefix_scratch(false) * most))) ||
-      (rc = ws.head_jobs.reserve(sizeof(PrefixJob) * nj)) ||
-      (rc = ws.head_res.reserve(sizeof(PrefixResult) * nj)))
+  if ((rc = ws.head_jobs.reserve(sizeof(PrefixJob) * nj)) || (rc = ws.head_res.reserve(sizeof(PrefixResult) * nj)))
     return rc;
+  const size_t most = std::max(nreal, nj - nreal);
+  size_t chunk = std::min<size_t>(most, std::max(sm_count(device), 1));
+  for (;; chunk = (chunk + 1) / 2) {
+    rc = ws.head.reserve(std::max(nreal ? prefix_scratch(true, lists[1]) * std::min(nreal, chunk) : 0,
+                                  nreal < nj ? prefix_scratch(false, lists[0]) * std::min(nj - nreal, chunk) : 0));
+    if (!rc) break;
+    cudaGetLastError();
+    if (chunk == 1) return rc;
+  }
   cudaError_t e = cudaFuncSetAttribute(kpm_prefix<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)prefix_smem(true));
   if (e == cudaSuccess)
@@ -415,10 +428,10 @@ static int run_fp64_head(cudaStream_t st, const std::vector<PrefixJob> &jobs, Wo
   uint64_t launches = 0;
   for (size_t j0 = 0; j0 < nj; launches++) {
     const bool real = j0 < nreal;
-    const size_t n = std::min<size_t>((real ? nreal : nj) - j0, kPrefixMaxJobs);
+    const size_t n = std::min((real ? nreal : nj) - j0, chunk);
     auto kern = real ? kpm_prefix<true> : kpm_prefix<false>;
     kern<<<(unsigned)n, kPrefixBlock, prefix_smem(real), st>>>(ws.head_jobs.as<PrefixJob>() + j0, ws.head.as<char>(),
-                                                               ws.head_res.as<PrefixResult>() + j0);
+                                                               lists[real], ws.head_res.as<PrefixResult>() + j0);
     j0 += n;
   }
   count_launches(launches);

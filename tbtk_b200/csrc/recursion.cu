@@ -500,7 +500,7 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
       j.width = m->widest_slice;
     }
     std::vector<PrefixResult> res;
-    if ((rc = run_fp64_head(st, jobs, ws, res))) return rc;
+    if ((rc = run_fp64_head(st, m->device, jobs, ws, res))) return rc;
     q = want;
     for (const PrefixResult &r : res) q = std::min(q, r.q);
     if (q < want) {
@@ -511,7 +511,7 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
         return cuda_fail(e, "recursion: staging");
       if (q >= 2) {
         for (PrefixJob &j : jobs) j.steps = q;
-        if ((rc = run_fp64_head(st, jobs, ws, res))) return rc;
+        if ((rc = run_fp64_head(st, m->device, jobs, ws, res))) return rc;
       } else {
         q = 0;  // the moment rows the head touched are rewritten by the plain start
       }

@@ -832,7 +832,7 @@ int run_joins(tbtkkpm_server *s, const std::vector<MultiJoin> &joins, const std:
     which.push_back(i);
   }
   std::vector<PrefixResult> res;
-  if ((rc = run_fp64_head(st, jobs, s->head_ws, res))) return rc;
+  if ((rc = run_fp64_head(st, s->device, jobs, s->head_ws, res))) return rc;
   for (size_t k = 0; k < which.size(); k++) head[which[k]] = res[k].q >= 2 ? res[k].q : 0;
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "server: joins");
   return TBTKKPM_OK;
