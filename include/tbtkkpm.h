@@ -112,6 +112,9 @@ TBTKKPM_API int tbtkkpm_matrix_create_triplets(
 	const uint32_t *rows, const uint32_t *cols, const double *vals,
 	uint64_t n, uint32_t N, double scale, tbtkkpm_matrix **out);
 
+/* Device memory of a destroyed matrix or table serves later handles: blocks of
+ * up to 64 MB, 256 MB a device at most, are kept until the last matrix and
+ * table is destroyed or an allocation of the library fails. */
 TBTKKPM_API int tbtkkpm_matrix_destroy(tbtkkpm_matrix *m);
 
 /* Runs this handle's work on the caller's CUDA stream (a cudaStream_t of
@@ -434,8 +437,9 @@ TBTKKPM_API int tbtkkpm_expectation_values(
  * a request whose model does not fit waits.  Outside the budget lie the
  * matrices, the tables and the scratch of the FP64 head: 0.06 MB (real) or
  * 0.11 MB (complex) an entry of the widest row, up to 10, and 0.3 MB more for a
- * complex model, for each lane that starts, of at most one per SM at once.  Any thread may submit and
- * wait; one worker thread per server drives the device. */
+ * complex model, for each lane that starts, of at most one per SM at once.
+ * Any thread may submit and wait; one worker thread per server drives the
+ * device. */
 
 typedef struct tbtkkpm_server tbtkkpm_server;
 
@@ -577,7 +581,8 @@ TBTKKPM_API int tbtkkpm_server_set_table_free(tbtkkpm_server *s, int enable);
  * (many lane classes of small models) replays a CUDA graph of one step of
  * every lane class, captured when the tick starts (a device counter gives each
  * replay its step); enable = 0 launches every kernel of every step directly.
- * A capture that fails turns graphs off for the server.  Results do not depend on it.  (No reference counterpart.) */
+ * A capture that fails turns graphs off for the server.  Results do not depend
+ * on it.  (No reference counterpart.) */
 TBTKKPM_API int tbtkkpm_server_set_graphs(tbtkkpm_server *s, int enable);
 
 /* enable = 1 (the default): a model steps at the narrowest width (a power

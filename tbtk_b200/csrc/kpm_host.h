@@ -50,8 +50,8 @@ struct DevBuf {
   template <typename T> T *as() const { return static_cast<T *>(ptr); }
 };
 
-// Counts a handle (matrix, table, server) for the block cache, which is
-// emptied when the last one goes.
+// Counts a handle (matrix, table) for the block cache, which is emptied when
+// the last one goes.
 void cache_handle_added();
 void cache_handle_removed();
 
@@ -85,8 +85,8 @@ struct Workspace {
   DevBuf damp;        // [M] damping numerators
   DevBuf out;         // results ([B][E] LDOS)
   DevBuf mu_direct;   // [K][steps+1] directly gathered moments (doubling runs)
-  DevBuf dots;        // [grid][2][Bp] per-block dot products (doubling runs), or the
-                      // warps' sums of an on-chip run
+  DevBuf dots;        // [steps][grid][2][Bp] per-block dot products of up to 64 steps
+                      // (doubling runs), or the blocks' sums of an on-chip run
   DevBuf col_out;     // [Bp] output slot of each batch column (doubling runs)
   DevBuf err;         // device flag of a bounded wait that ran out
   DevBuf head, head_jobs, head_res;  // FP64 head of doubling runs (scratch, jobs, results)

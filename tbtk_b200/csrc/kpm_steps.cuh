@@ -186,8 +186,9 @@ void launch_async(cudaStream_t st, int device, unsigned max_grid, const StepArgs
 // warps, BPS blocks per SM).
 constexpr int kTiledVariant = 100000;
 constexpr int kTiledReal64 = 200;
-// Columns staged together: the copies move multiples of 16 bytes, so rows of
-// 8 and 4 bytes go two and four at a time.
+// Fewest columns a copy may take: the copies move multiples of 16 bytes, so
+// rows of 8 and 4 bytes need plans of at least two and four columns staged
+// together (built are one and four).
 constexpr uint32_t tiled_unit(uint32_t rowbytes) { return rowbytes >= 16 ? 1 : 16 / rowbytes; }
 inline bool is_tiled_variant(int v) { return v >= kTiledVariant; }
 inline int tiled_rows(int v) { return ((v - kTiledVariant) % 1000000) / 1000; }

@@ -671,9 +671,10 @@ kpm_step_tiled(TilePlan P, TiledLayout LY, uint32_t Bp,
 // the runs of consecutive ones counted (k_plan_count) or listed
 // (k_plan_fill).  A tile with more than kPlanCap entries sets *bad.
 
-// UNIT is the number of columns staged together: 1, or 2 or 4 for vector rows
-// of 8 or 4 bytes, whose copies would otherwise break the 16-byte rule.  A unit is
-// the columns [UNIT*i, UNIT*(i + 1)); runs and slots are in columns.
+// UNIT is the number of columns staged together: 1, or 4 for vector rows of 8
+// or 4 bytes, whose copies would otherwise break the 16-byte rule, and where
+// it saves copies (fitting_plan).  A unit is the columns [UNIT*i, UNIT*(i + 1));
+// runs and slots are in columns.
 
 // Loads the units of the tile's outside columns (each by its first column)
 // into keys[0, n2) (n2 = next power of two of the entry count, padded with

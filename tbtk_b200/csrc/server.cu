@@ -10,8 +10,9 @@
 //   tick   - joins (column = e_source, or an FP64 head), then S steps of
 //            every lane class (width, real or complex lanes) over all
 //            models with busy lanes, S ending no later than the first lane
-//            that finishes: one step of every class captured as a CUDA
-//            graph and replayed S times, the classes on their own streams;
+//            that finishes, the classes on their own streams, as dependent
+//            launches, or where those take longer than the steps as a CUDA
+//            graph of one step of every class replayed S times;
 //   finish - for every finished request: moments damped and summed over the
 //            energy grid on the device (LDOS or the request's Green's
 //            function type), the error estimate, release of the lanes.
@@ -364,8 +365,9 @@ struct tbtkkpm_server {
   static constexpr int kClassStreams = 4;
   cudaStream_t cls_stream[kClassStreams] = {};
   cudaEvent_t ev_fork = nullptr, ev_join[kClassStreams] = {};
-  // Each tick's steps replay a captured CUDA graph of one step of every
-  // class (tick_exec; d_step counts the replays); off when a capture failed.
+  // Ticks of short steps replay a captured CUDA graph of one step of every
+  // class (run_tick; tick_exec, d_step counts the replays); off when a
+  // capture failed.
   bool use_graphs = true;
   cudaGraphExec_t tick_exec = nullptr;
   DevBuf d_step;
