@@ -107,6 +107,7 @@ struct TilePlan {
   uint32_t N, ntiles, R;
   uint32_t umax, wmax;     // most distinct outside columns / entries per row of a tile
   uint32_t nruns;          // runs of all tiles
+  uint64_t staged, slots;  // outside columns staged / entry slots of all tiles
   uint32_t pairs;          // row-pair plan: entries of [w][R/2] row pairs, two values each
   uint32_t unit;           // columns staged together (1 or 4)
 };

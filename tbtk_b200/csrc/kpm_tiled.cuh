@@ -782,6 +782,7 @@ k_plan_count(uint32_t N, uint32_t ntiles, const uint32_t *__restrict__ rowptr,
       tw[t] = cnt[2];
       atomicMax(&maxes[0], cnt[0] * UNIT);
       atomicMax(&maxes[1], cnt[2]);
+      atomicAdd(reinterpret_cast<unsigned long long *>(maxes + 4), (unsigned long long)(cnt[0] * UNIT));
     }
     __syncthreads();
   }

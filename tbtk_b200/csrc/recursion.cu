@@ -310,25 +310,88 @@ int fitting_plan(tbtkkpm_matrix *m, const StepEntry *fn, const TilePlan *&plan) 
   return TBTKKPM_OK;
 }
 
+// Microseconds of a tile-staged step with plan p: launch and round trips, the
+// copies that a producer warp issues one by one, the rows and entries moved,
+// and a consumer's serial entries.  Fitted, like register_us, to 2112 batches of
+// 1 to 128 sources on 66 matrices of 11k to 500k rows: square, Rashba,
+// honeycomb and cubic lattices, bands, and lattices whose rows are renumbered at
+// random, in all or within windows of 16, 128 and 1024 rows.  Nine in ten times
+// within 25%.
+double tiled_us(const StepEntry *e, const TilePlan &p, int device) {
+  // us, us per copy and round, us per MB staged and MB of entries, us per entry
+  struct Fit { double fixed, run, staged, entries, serial; };
+  static const Fit fits[6] = {{2.4, 0.033, 0.037, 0.093, 0.046}, {2.3, 0.028, 0.015, 0.062, 0.049},
+                              {2.9, 0.028, 0.024, 0.064, 0.050}, {2.5, 0.034, 0.025, 0.062, 0.025},
+                              {3.2, 0.034, 0.051, 0.063, 0.025}, {2.6, 0.032, 0.042, 0.110, 0.013}};
+  const Fit &f = fits[e->cls];
+  const double esz = e->cls == kClassFP64 ? 16 : e->cls == kClassMixedReal || e->cls == kClassMixedRealDots ? 4 : 8;
+  const double vsz = e->cls <= kClassMixedDots ? 16 : 8;
+  const double grid = std::min<double>(p.ntiles, (double)tiled_bps(e->minb) * sm_count(device));
+  const double rounds = std::ceil(p.ntiles / grid), tiles = p.ntiles;
+  const double passes = std::ceil((double)p.R * e->tpr / (32.0 * tiled_warps(e->minb)));
+  return f.fixed + f.run * rounds * p.nruns / tiles +
+         f.staged * 1e-6 * (p.staged + 2.0 * p.R * tiles) * e->tpr * e->vpt * esz +
+         f.entries * 1e-6 * p.slots * (vsz + 2) +
+         f.serial * rounds * passes * (p.slots / (p.R * tiles)) * e->vpt;
+}
+
+// The same of the register-staged default of a batch of padded width Bp (cls:
+// its class): entries, bytes gathered and moved, and how its shape does
+// against that of one source.  Nine in ten times within 27%.
+double register_us(const tbtkkpm_matrix *m, int cls, uint32_t Bp) {
+  struct Fit { double fixed, entry, gather, move, shape[8]; };  // us, us per 1e6 entries, us per MB
+  static const Fit fits[5] = {
+      {4.3, 0.0, 0.190, 1.30, {1, 1.22, 1.02, 0.97, 0.83, 0.78, 0.48, 0.39}},
+      {6.0, 1.1, 0.240, 1.20, {1, 0.82, 0.76, 0.90, 0.89, 0.63, 0.55, 0.49}},
+      {7.7, 1.2, 0.180, 1.20, {1, 1.10, 1.13, 1.02, 1.06, 0.84, 0.77, 0.71}},
+      {4.7, 2.3, 0.120, 0.78, {1, 0.98, 1.05, 0.96, 1.16, 1.05, 0.91, 0.89}},
+      {7.0, 2.1, 0.038, 0.32, {1, 1.22, 1.63, 2.36, 3.59, 2.92, 2.28, 2.12}}};
+  const Fit &f = fits[cls];
+  const double rowbytes = Bp * (cls == kClassFP64 ? 16.0 : cls <= kClassMixedDots ? 8.0 : 4.0);
+  int i = 0;
+  while (i < 7 && (1u << i) < Bp) i++;
+  return f.shape[i] *
+         (f.fixed + 1e-6 * (f.entry * m->nnz + (f.gather * m->nnz + f.move * m->N) * rowbytes));
+}
+
+// Whether the register-staged default is the better one.  Without locality a
+// tile needs a copy per entry and stages rows for one use each: randomly
+// numbered square sites, 125k rows, two real sources of directly gathered
+// moments: 70 us a step tile-staged, 8 register-staged.  The rule's choice is
+// within 0.3% of the faster on average over those batches, at most 1.5 times
+// it, and always tile-staged on the lattices (at most 0.85 of the estimates).
+bool register_wins(const tbtkkpm_matrix *m, const StepEntry *e, const TilePlan &p) {
+  const int cls = e->cls == kClassFP64Real ? (int)kClassFP64 : e->cls;
+  return tiled_us(e, p, m->device) > 1.05 * register_us(m, cls, (uint32_t)(e->tpr * e->vpt));
+}
+
 // A tile-staged entry runs with a plan that fits (fitting_plan); one on real
-// FP64 vectors also needs the batch to take them (real64).  Otherwise a
-// forced entry is refused (TBTKKPM_ERR_UNSUPPORTED, which the autotuner
-// skips) and a chosen one gives way: to the tile-staged entry of its class
+// FP64 vectors also needs the batch to take them (real64).  A default, not
+// `chosen` by set_config or the autotuner, also has to be worth it
+// (register_wins).  Otherwise a forced entry is refused
+// (TBTKKPM_ERR_UNSUPPORTED, which the autotuner skips) and any other one gives
+// way: to the tile-staged entry of its class
 // and width that fits with the most consumer warps per SM (wide rows: on the
 // 512^2 Rashba lattice one FP64 source takes 16 us per step with 6 blocks per
 // SM, where 8 do not fit, against 30 register-staged), then real FP64 vectors
 // to the complex default, then to the register-staged default of the batch.
-int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool forced, bool real64,
-                  const StepEntry *&fn, const TilePlan *&plan) {
+int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool forced, bool chosen,
+                  bool real64, const StepEntry *&fn, const TilePlan *&plan) {
   plan = nullptr;
   const bool real = real_mode(m, precision);
   const int cls = step_class(precision, dots, real);
   int rc;
+  auto registers = [&]() {
+    plan = nullptr;
+    const Shape s = register_shape_for(precision, B, real, dots);
+    fn = find_step(cls, s.tpr, s.vpt, s.minb);
+  };
   while (fn && is_tiled_variant(fn->minb)) {
     const bool r64 = fn->cls == kClassFP64Real;
     if (!r64 || real64) {
       if ((rc = fitting_plan(m, fn, plan))) return rc;
-      if (plan) return TBTKKPM_OK;
+      if (plan && !forced && !chosen && register_wins(m, fn, *plan)) registers();
+      if (plan || !is_tiled_variant(fn->minb)) return TBTKKPM_OK;
     }
     if (forced)
       return fail(TBTKKPM_ERR_UNSUPPORTED,
@@ -350,13 +413,18 @@ int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool 
         if ((rc = fitting_plan(m, e, plan))) return rc;
         if (plan) {
           fn = e;
+          if (register_wins(m, fn, *plan)) registers();
           return TBTKKPM_OK;
         }
       }
     }
-    const Shape s = r64 ? shape_for(precision, B, false, dots, m->N, m->widest_slice)
-                        : register_shape_for(precision, B, real, dots);
-    fn = find_step(cls, s.tpr, s.vpt, s.minb);
+    if (r64) {
+      const Shape s = shape_for(precision, B, false, dots, m->N, m->widest_slice);
+      fn = find_step(cls, s.tpr, s.vpt, s.minb);
+      chosen = false;
+    } else {
+      registers();
+    }
   }
   return TBTKKPM_OK;
 }
@@ -402,8 +470,9 @@ int run_batch(tbtkkpm_matrix *m, int precision, const std::vector<uint32_t> &fro
                                  (uint32_t)tl.row.size(), res))) return rc;
   const TilePlan *plan = nullptr;
   if (!res.ok) {
+    const bool chosen = fn != nullptr;
     if (!fn) fn = default_step(m, precision, doubling, B, real64);
-    if ((rc = resolve_tiled(m, precision, doubling, B, force != nullptr, real64, fn, plan))) return rc;
+    if ((rc = resolve_tiled(m, precision, doubling, B, force != nullptr, chosen, real64, fn, plan))) return rc;
     if (!fn) return fail(TBTKKPM_ERR_UNSUPPORTED, "no recursion kernel for batch %u", B);
     kind = fn->cls == kClassFP64 ? kVecF64C : fn->cls == kClassFP64Real ? kVecF64R
            : fn->cls == kClassMixedReal || fn->cls == kClassMixedRealDots ? kVecF32 : kVecC64;

@@ -70,10 +70,10 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, T
   int rc;
   if ((rc = tw.reserve(4 * ((size_t)ntiles + 1))) || (rc = truns.reserve(4 * ((size_t)ntiles + 1))) ||
       (rc = tuniq.reserve(4 * ((size_t)ntiles + 1))) || (rc = ent.reserve(4 * ((size_t)ntiles + 1))) ||
-      (rc = run.reserve(4 * ((size_t)ntiles + 1))) || (rc = flags.reserve(16)))
+      (rc = run.reserve(4 * ((size_t)ntiles + 1))) || (rc = flags.reserve(24)))
     return rc;
   cudaError_t e;
-  if ((e = cudaMemsetAsync(flags.ptr, 0, 16, st)) ||
+  if ((e = cudaMemsetAsync(flags.ptr, 0, 24, st)) ||
       (e = cudaMemsetAsync(tw.as<uint32_t>() + ntiles, 0, 4, st)) ||
       (e = cudaMemsetAsync(truns.as<uint32_t>() + ntiles, 0, 4, st)))
     return cuda_fail(e, "tile plan: staging");
@@ -92,9 +92,10 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, T
     count_launches(1);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "tile plan: pairs");
   }
-  // most distinct outside columns, widest row, a tile too large, widest pair merge
-  unsigned hf[4] = {0, 0, 0, 0};
-  if ((e = cudaMemcpyAsync(hf, flags.ptr, 16, cudaMemcpyDeviceToHost, st)) ||
+  // most distinct outside columns, widest row, a tile too large, widest pair
+  // merge; distinct outside columns of all tiles (64 bits)
+  unsigned hf[6] = {0, 0, 0, 0, 0, 0};
+  if ((e = cudaMemcpyAsync(hf, flags.ptr, 24, cudaMemcpyDeviceToHost, st)) ||
       (e = cudaStreamSynchronize(st)))
     return cuda_fail(e, "tile plan: count");
   if (pairs) hf[1] = hf[3];
@@ -145,6 +146,8 @@ int build_plan(tbtkkpm_matrix *m, int R, bool cplx, bool pairs, uint32_t unit, T
   p.plan.umax = hf[0];
   p.plan.wmax = hf[1];
   p.plan.nruns = nruns;
+  p.plan.staged = (uint64_t)hf[5] << 32 | hf[4];
+  p.plan.slots = slots;
   p.plan.pairs = pairs ? 1u : 0u;
   p.plan.unit = unit;
   p.ok = true;
