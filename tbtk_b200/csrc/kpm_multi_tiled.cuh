@@ -437,21 +437,31 @@ kpm_multi_tiled(const MultiModel *__restrict__ models, const MultiHeader *__rest
       if (lane == 0) mbar_arrive(&empty[s]);
     }
     // The last sums go over the block's warps through the ring (every warp has
-    // used its last stage; after a wait that ran out the step's results are
-    // dropped), then one atomic per column and block: atomics on the same few
-    // addresses go one by one in L2 (16 lanes of a 74k-row model: 11.5 us a
-    // step, with one atomic per column and warp 27.5).
+    // used its last stage), then one atomic per column and block: atomics on the
+    // same few addresses go one by one in L2 (16 lanes of a 74k-row model: 11.5
+    // us a step, with one atomic per column and warp 27.5).  After a wait that
+    // ran out in any warp copies may still land in the ring and a warp may have
+    // no model to add to: the sums of the step, whose results are dropped, are
+    // left out.
     static_assert(R >= CW, "the warps' sums fit two stages of the ring");
     constexpr uint32_t kThreads = CW * 32;
-    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
-    long long *red = reinterpret_cast<long long *>(ring);
-    flush([&](uint32_t c, long long v) { red[(uint32_t)(warp - 1) * 2 * W + c] = v; });
-    asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
-    for (uint32_t c = (uint32_t)ct; c < 2 * W; c += kThreads) {
-      long long v = 0;
+    uint32_t any_failed;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(any_failed)
+        : "r"(failed ? 1u : 0u), "n"(kThreads)
+        : "memory");
+    if (!any_failed) {
+      long long *red = reinterpret_cast<long long *>(ring);
+      flush([&](uint32_t c, long long v) { red[(uint32_t)(warp - 1) * 2 * W + c] = v; });
+      asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+      for (uint32_t c = (uint32_t)ct; c < 2 * W; c += kThreads) {
+        long long v = 0;
 #pragma unroll
-      for (int u = 0; u < CW; u++) v += red[(uint32_t)u * 2 * W + c];
-      add(c, v);
+        for (int u = 0; u < CW; u++) v += red[(uint32_t)u * 2 * W + c];
+        add(c, v);
+      }
     }
     if (failed && lane == 0) atomicExch(err, kErrTimeout);
   }
