@@ -370,11 +370,13 @@ bool register_wins(const tbtkkpm_matrix *m, const StepEntry *e, const TilePlan &
 // `chosen` by set_config or the autotuner, also has to be worth it
 // (register_wins).  Otherwise a forced entry is refused
 // (TBTKKPM_ERR_UNSUPPORTED, which the autotuner skips) and any other one gives
-// way: to the tile-staged entry of its class
-// and width that fits with the most consumer warps per SM (wide rows: on the
+// way: to the tile-staged entry of its class and width that fits, one of the
+// same threads and values per row first (32 FP64 sources on the 500^2 Rashba
+// lattice, whose 32-row tiles do not fit: 172 us in 16-row tiles of (16, 2),
+// 238 in those of (32, 1)), then by consumer warps per SM (wide rows: on the
 // 512^2 Rashba lattice one FP64 source takes 16 us per step with 6 blocks per
-// SM, where 8 do not fit, against 30 register-staged), then real FP64 vectors
-// to the complex default, then to the register-staged default of the batch.
+// SM, where 8 do not fit, against 30 register-staged); then real FP64 vectors
+// to the complex default; then to the register-staged default of the batch.
 int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool forced, bool chosen,
                   bool real64, const StepEntry *&fn, const TilePlan *&plan) {
   plan = nullptr;
@@ -401,14 +403,17 @@ int resolve_tiled(tbtkkpm_matrix *m, int precision, bool dots, uint32_t B, bool 
       const StepEntry *t;
       int n;
       step_table(cls, &t, &n);
+      const StepEntry &shape = *fn;
       std::vector<const StepEntry *> others;
       for (int i = 0; i < n; i++)
         if (&t[i] != fn && t[i].cls == fn->cls && t[i].tpr * t[i].vpt == fn->tpr * fn->vpt &&
             is_tiled_variant(t[i].minb) && !tiled_pairs(t[i].minb))
           others.push_back(&t[i]);
       auto warps = [](const StepEntry *e) { return tiled_bps(e->minb) * tiled_warps(e->minb); };
-      std::stable_sort(others.begin(), others.end(),
-                       [&](const StepEntry *a, const StepEntry *b) { return warps(a) > warps(b); });
+      auto alike = [&](const StepEntry *e) { return e->tpr == shape.tpr && e->vpt == shape.vpt; };
+      std::stable_sort(others.begin(), others.end(), [&](const StepEntry *a, const StepEntry *b) {
+        return alike(a) != alike(b) ? alike(a) : warps(a) > warps(b);
+      });
       for (const StepEntry *e : others) {
         if ((rc = fitting_plan(m, e, plan))) return rc;
         if (plan) {
