@@ -22,3 +22,30 @@ def test_same_shape_in_smaller_tiles(gpu, name, L, B, kind):
     ms = [_ms(gpu, m, kind, sites) for m in (a, b)]
     assert ms[0] <= 1.1 * ms[1], ms
     assert np.array_equal(_call(gpu, a, kind, sites), _call(gpu, b, kind, sites))
+
+
+def _band(N, reach):
+    i = np.repeat(np.arange(N), 2 * reach + 1)
+    j = i + np.tile(np.arange(-reach, reach + 1), N)
+    i, j = i[(j >= 0) & (j < N)], j[(j >= 0) & (j < N)]
+    rp = np.concatenate([[0], np.cumsum(np.bincount(i, minlength=N))])
+    return rp.astype(np.uint32), j.astype(np.uint32), 0.2 * np.cos(i + j) + 0j
+
+
+@pytest.mark.parametrize("kind", ["ldos_fp64", "moments_fp64"])
+@pytest.mark.parametrize("N,B,config", [(20000, 1, (1, 1)), (20000, 2, (2, 1)), (60001, 1, (1, 1))])
+def test_wide_rows_build_no_plans(gpu, N, B, config, kind):
+    """Rows of 31 entries leave one or two FP64 sources no ring: the first call
+    by default launches what it does with the register-staged step set."""
+    csr = _band(N, 15)
+    sites = (np.arange(B) * (N // B)).astype(np.uint32)
+    n = []
+    for c in (None, config):
+        m = gpu.Matrix.from_csr(*csr, SCALE)
+        m.set_wait_limit(1 << 22)  # launched steps
+        if c:
+            m.set_config(B, gpu.FP64, *c, 2, ldos=kind.startswith("ldos"))
+        n.append(-gpu.kernel_launches())
+        _call(gpu, m, kind, sites)
+        n[-1] += gpu.kernel_launches()
+    assert n[0] == n[1]
