@@ -161,8 +161,11 @@ struct tbtkkpm_matrix {
   uint64_t chunks = 0;
   uint32_t widest_slice = 0;  // entries of the longest row
   // on-chip recursion (resident.cu), filled on first use: slice_ptr on the
-  // host, groups at once per (kernel shape, shared memory)
+  // host, groups at once per (kernel shape, shared memory), the matrix's
+  // locality: shares of its entries that are scattered, and that lie with
+  // another of 1, 2, ... 16 blocks, scattered or next to the row before's
   std::vector<uint32_t> host_slice_ptr;
+  double scattered = 0, far_scattered[5] = {0}, far_next[5] = {0};
   std::map<uint64_t, uint32_t> resident_groups;
   tbtkkpm::Workspace ws;
   tbtkkpm::PhaseTimer timer;
@@ -240,6 +243,8 @@ struct ResidentPlan {
   uint32_t cluster = 1, cols = 1, groups = 0, warps = 1, spb = 0, chunks = 0, cap = 0;
   size_t smem = 0;
 };
+// Estimated us of a register-staged default step (recursion.cu).
+double register_us(const tbtkkpm_matrix *m, int cls, uint32_t Bp);
 struct ResidentArgs;
 constexpr uint32_t kResMaxSlices = 4096;
 int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint32_t *trow,

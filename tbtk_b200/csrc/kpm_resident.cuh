@@ -525,6 +525,38 @@ kpm_resident(ResidentArgs R) {
   }
 }
 
+// Locality of a matrix's entries for the estimates of resident.cu: out[0] those
+// not within two columns of the row before's entry of the same place,
+// out[1 + 2c] those of them and out[2 + 2c] the others that another block owns
+// when 2^c blocks share the slices.  A warp per slice.
+static __global__ void __launch_bounds__(256)
+k_locality(Sell A, uint32_t *out) {
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (s >= A.nslices) return;
+  const uint32_t k0 = __ldg(A.slice_ptr + s), k1 = __ldg(A.slice_ptr + s + 1);
+  uint32_t n[11];
+#pragma unroll
+  for (int i = 0; i < 11; i++) n[i] = 0;
+  for (uint32_t k = k0; k < k1; k++) {
+    const uint32_t c = __ldg(A.col + (uint64_t)k * 32 + lane);
+    const uint32_t before = __shfl_up_sync(0xffffffffu, c, 1);
+    const bool live = c != kPad;
+    const bool scattered = lane == 0 || before == kPad || c + 2 < before || c > before + 2;
+    n[0] += __popc(__ballot_sync(0xffffffffu, live && scattered));
+#pragma unroll
+    for (int i = 0; i < 5; i++) {
+      const uint32_t spb = (A.nslices + (1u << i) - 1) >> i;
+      const bool away = live && (c >> 5) / spb != s / spb;
+      n[1 + 2 * i] += __popc(__ballot_sync(0xffffffffu, away && scattered));
+      n[2 + 2 * i] += __popc(__ballot_sync(0xffffffffu, away && !scattered));
+    }
+  }
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < 11; i++)
+      if (n[i]) atomicAdd(out + i, n[i]);
+}
+
 // The doubled moments of steps n0.. from the blocks' sums of kpm_resident (as
 // kpm_dots_finalize): one warp per (step, column), the sums in a fixed order.
 static __global__ void __launch_bounds__(256)

@@ -344,6 +344,8 @@ double tiled_us(const StepEntry *e, const TilePlan &p, int device) {
          f.serial * rounds * passes * (p.slots / (p.R * tiles)) * e->vpt;
 }
 
+}  // namespace
+
 // The same of the register-staged default of a batch of padded width Bp (cls:
 // its class): entries, bytes gathered and moved, and how its shape does
 // against that of one source.  Nine in ten times within 27%.
@@ -362,6 +364,8 @@ double register_us(const tbtkkpm_matrix *m, int cls, uint32_t Bp) {
   return f.shape[i] *
          (f.fixed + 1e-6 * (f.entry * m->nnz + (f.gather * m->nnz + f.move * m->N) * rowbytes));
 }
+
+namespace {
 
 // Whether the register-staged default is the better one.  Without locality a
 // tile needs a copy per entry and stages rows for one use each: randomly

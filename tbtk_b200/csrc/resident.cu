@@ -124,7 +124,12 @@ static uint32_t resident_groups(const ResidentPlan &p, int device) {
 // blocks share an SM, and the doubling sums.  Measured for FP64 real / complex,
 // one source: 0.65 / 0.83 us at 512 rows, 0.74 / 0.93 at 1800, 0.80 / 1.2 at
 // 8192; a batch of 128 sources of 1800 rows 2.1 / 4.3.
-static double wave_us(const ResidentPlan &p, uint32_t groups_at_once, uint32_t sms) {
+// A load from another block costs 1.3 ns a block and SM where the lanes of a
+// warp reach scattered rows, a tenth of that where they reach neighbours
+// (measured on the same lattices with their rows renumbered at random, where
+// the estimate without it was a quarter of the time: 11k rows of 9 entries 11.2
+// us a step, launched 6.2).
+static double wave_us(const tbtkkpm_matrix *m, const ResidentPlan &p, uint32_t groups_at_once, uint32_t sms) {
   static const double base[2][4] = {{0.74, 0.45, 0.45, 0.52}, {0.49, 0.34, 0.64, 0.35}};
   static const double entry_ns[2][4] = {{0.168, 0.129, 0.205, 0.135}, {0.122, 0.044, 0.073, 0.044}};
   static const double wider[2][2] = {{1.26, 1.88}, {1.87, 3.78}};  // two and four columns
@@ -138,6 +143,9 @@ static double wave_us(const ResidentPlan &p, uint32_t groups_at_once, uint32_t s
               column[p.kind] * (p.cols - 1);
   if (p.dots) us += 0.18 * (1 + 0.4 * (p.cols - 1));
   if (p.cap == 0) us += 1.2;  // moments stored step by step
+  int c = 0;
+  while ((1u << c) < p.cluster) c++;
+  us += 1e-3 * m->nnz / p.cluster * (1.3 * m->far_scattered[c] + 0.13 * m->far_next[c]) * std::max(blocks, 1.0);
   return us * ((p.groups + groups_at_once - 1) / groups_at_once);
 }
 
@@ -154,8 +162,17 @@ static double launch_us(const tbtkkpm_matrix *m, int kind, bool dots, uint32_t B
   const Fit &f = dots ? doubled[kind - kVecC64] : direct[kind];
   int log2w = 0;
   while ((1u << log2w) < B) log2w++;
-  return f.fixed + f.doubling * log2w +
-         1e-6 * (double)(1u << log2w) * (f.row * m->N + f.entry * 32.0 * m->chunks);
+  const double us = f.fixed + f.doubling * log2w +
+                    1e-6 * (double)(1u << log2w) * (f.row * m->N + f.entry * 32.0 * m->chunks);
+  // Scattered entries and long rows, which those lattices do not have, bring
+  // it towards the register-staged step's, not all the way, since few batches
+  // should leave the launched step for a slower one (6 of 575 do by more than a
+  // tenth, at most 1.6 times; of 575 the choice is 3 to 8% from the better path on
+  // average).
+  const double share = std::max((m->scattered - 0.4) / 0.5, ((double)m->nnz / m->N - 10) / 20);
+  if (share <= 0) return us;
+  const int cls = kind <= kVecF64R ? 0 : kind == kVecC64 ? 1 + dots : 3 + dots;
+  return us + 0.8 * std::min(share, 1.0) * std::max(register_us(m, cls, 1u << log2w) - us, 0.0);
 }
 
 int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint32_t *trow,
@@ -166,10 +183,33 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
   if (m->wait_limit != TBTKKPM_WAIT_DEFAULT) return TBTKKPM_OK;
   if (m->host_slice_ptr.size() != (size_t)m->nslices + 1) {
     std::vector<uint32_t> sp((size_t)m->nslices + 1);
-    cudaError_t e = cudaMemcpyAsync(sp.data(), m->slice_ptr.ptr, 4 * sp.size(), cudaMemcpyDeviceToHost,
-                                    m->stream);
+    ScratchBufs<1> scratch(m->stream);
+    DevBuf &n = scratch.b[0];
+    uint32_t hn[11];
+    int rc = n.reserve(sizeof hn);
+    if (rc) return rc;
+    Sell A{};
+    A.slice_ptr = m->slice_ptr.as<uint32_t>();
+    A.col = m->scol.as<uint32_t>();
+    A.N = m->N;
+    A.nslices = m->nslices;
+    cudaError_t e = cudaMemsetAsync(n.ptr, 0, sizeof hn, m->stream);
+    if (e == cudaSuccess) {
+      k_locality<<<(m->nslices + 7) / 8, 256, 0, m->stream>>>(A, n.as<uint32_t>());
+      count_launches(1);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(sp.data(), m->slice_ptr.ptr, 4 * sp.size(), cudaMemcpyDeviceToHost, m->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hn, n.ptr, sizeof hn, cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) return cuda_fail(e, "recursion: slice bounds");
+    const double all = (double)std::max<uint64_t>(m->nnz, 1);
+    m->scattered = hn[0] / all;
+    for (int i = 0; i < 5; i++) {
+      m->far_scattered[i] = hn[1 + 2 * i] / all;
+      m->far_next[i] = hn[2 + 2 * i] / all;
+    }
     m->host_slice_ptr = std::move(sp);
   }
   // Below the launched step by a margin for the error of both estimates.  Over
@@ -188,7 +228,7 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
       p.cols = cols;
       p.groups = (B + cols - 1) / cols;
       if (!shape_resident(m, trow, tcol, T, p)) continue;
-      if (wave_us(p, p.groups, p.groups * p.cluster) >= best) continue;  // at least that
+      if (wave_us(m, p, p.groups, p.groups * p.cluster) >= best) continue;  // at least that
       const uint64_t key = ((((uint64_t)kind * 2 + dots) * 32 + C) * 8 + cols) << 32 | p.smem;
       auto it = m->resident_groups.find(key);
       if (it == m->resident_groups.end()) {
@@ -196,7 +236,7 @@ int plan_resident(tbtkkpm_matrix *m, int kind, bool dots, uint32_t B, const uint
         it = m->resident_groups.emplace(key, resident_groups(p, m->device)).first;
       }
       if (it->second == 0) continue;
-      const double us = wave_us(p, it->second, (uint32_t)sm_count(m->device));
+      const double us = wave_us(m, p, it->second, (uint32_t)sm_count(m->device));
       if (us >= best) continue;
       best = us;
       p.ok = true;

@@ -22,11 +22,13 @@ def _ldos_launches(gpu, m, sites, precision):
     return _launches(gpu, lambda: m.ldos_sites(tab, sites, 1e-3, precision))
 
 
-@pytest.mark.parametrize("B", [1, 2, 12, 64, 128])
 @pytest.mark.parametrize("complex_", [False, True])
-@pytest.mark.parametrize("N", [1, 31, 100, 513, 1800])
-def test_small_matrices_run_on_chip(gpu, N, complex_, B):
-    """The sizes that test_resident compares with the step kernels."""
+@pytest.mark.parametrize("N,B", [(N, B) for N in (1, 31, 100, 513, 1800) for B in (1, 2, 12, 64, 128)
+                                 if N < 1800 or B < 64])
+def test_small_matrices_run_on_chip(gpu, N, B, complex_):
+    """Sizes that test_resident compares with the step kernels (1800 randomly
+    coupled rows of 64 and 128 FP64 sources are faster launched: 7.8 and 9.2 us a
+    step against 12 and 24)."""
     m = gpu.Matrix.from_csr(*_hermitian(N, 6, complex_, N), SCALE)
     sites = (np.arange(B) * 5 % N).astype(np.uint32)
     for p in (gpu.FP64, gpu.MIXED, gpu.MIXED_DIRECT):
