@@ -243,7 +243,9 @@ struct ResidentPlan {
   uint32_t cluster = 1, cols = 1, groups = 0, warps = 1, spb = 0, chunks = 0, cap = 0;
   size_t smem = 0;
 };
-// Estimated us of a register-staged default step (recursion.cu).
+// Estimated us of a tile-staged step (cls: StepClass; `warps` consumer warps,
+// `bps` blocks per SM) and of a register-staged default one (recursion.cu).
+double tiled_us(int cls, int tpr, int vpt, int warps, int bps, const TilePlan &p, int device);
 double register_us(const tbtkkpm_matrix *m, int cls, uint32_t Bp);
 struct ResidentArgs;
 constexpr uint32_t kResMaxSlices = 4096;

@@ -319,6 +319,8 @@ int fitting_plan(tbtkkpm_matrix *m, const StepEntry *fn, const TilePlan *&plan) 
   return TBTKKPM_OK;
 }
 
+}  // namespace
+
 // Microseconds of a tile-staged step with plan p: launch and round trips, the
 // copies that a producer warp issues one by one, the rows and entries moved,
 // and a consumer's serial entries.  Fitted, like register_us, to 2112 batches of
@@ -326,25 +328,23 @@ int fitting_plan(tbtkkpm_matrix *m, const StepEntry *fn, const TilePlan *&plan) 
 // honeycomb and cubic lattices, bands, and lattices whose rows are renumbered at
 // random, in all or within windows of 16, 128 and 1024 rows.  Nine in ten times
 // within 25%.
-double tiled_us(const StepEntry *e, const TilePlan &p, int device) {
+double tiled_us(int cls, int tpr, int vpt, int warps, int bps, const TilePlan &p, int device) {
   // us, us per copy and round, us per MB staged and MB of entries, us per entry
   struct Fit { double fixed, run, staged, entries, serial; };
   static const Fit fits[6] = {{2.4, 0.033, 0.037, 0.093, 0.046}, {2.3, 0.028, 0.015, 0.062, 0.049},
                               {2.9, 0.028, 0.024, 0.064, 0.050}, {2.5, 0.034, 0.025, 0.062, 0.025},
                               {3.2, 0.034, 0.051, 0.063, 0.025}, {2.6, 0.032, 0.042, 0.110, 0.013}};
-  const Fit &f = fits[e->cls];
-  const double esz = e->cls == kClassFP64 ? 16 : e->cls == kClassMixedReal || e->cls == kClassMixedRealDots ? 4 : 8;
-  const double vsz = e->cls <= kClassMixedDots ? 16 : 8;
-  const double grid = std::min<double>(p.ntiles, (double)tiled_bps(e->minb) * sm_count(device));
+  const Fit &f = fits[cls];
+  const double esz = cls == kClassFP64 ? 16 : cls == kClassMixedReal || cls == kClassMixedRealDots ? 4 : 8;
+  const double vsz = cls <= kClassMixedDots ? 16 : 8;
+  const double grid = std::min<double>(p.ntiles, (double)bps * sm_count(device));
   const double rounds = std::ceil(p.ntiles / grid), tiles = p.ntiles;
-  const double passes = std::ceil((double)p.R * e->tpr / (32.0 * tiled_warps(e->minb)));
+  const double passes = std::ceil((double)p.R * tpr / (32.0 * warps));
   return f.fixed + f.run * rounds * p.nruns / tiles +
-         f.staged * 1e-6 * (p.staged + 2.0 * p.R * tiles) * e->tpr * e->vpt * esz +
+         f.staged * 1e-6 * (p.staged + 2.0 * p.R * tiles) * tpr * vpt * esz +
          f.entries * 1e-6 * p.slots * (vsz + 2) +
-         f.serial * rounds * passes * (p.slots / (p.R * tiles)) * e->vpt;
+         f.serial * rounds * passes * (p.slots / (p.R * tiles)) * vpt;
 }
-
-}  // namespace
 
 // The same of the register-staged default of a batch of padded width Bp (cls:
 // its class): entries, bytes gathered and moved, and how its shape does
@@ -375,7 +375,8 @@ namespace {
 // it, and always tile-staged on the lattices (at most 0.85 of the estimates).
 bool register_wins(const tbtkkpm_matrix *m, const StepEntry *e, const TilePlan &p) {
   const int cls = e->cls == kClassFP64Real ? (int)kClassFP64 : e->cls;
-  return tiled_us(e, p, m->device) > 1.05 * register_us(m, cls, (uint32_t)(e->tpr * e->vpt));
+  const double us = tiled_us(e->cls, e->tpr, e->vpt, tiled_warps(e->minb), tiled_bps(e->minb), p, m->device);
+  return us > 1.05 * register_us(m, cls, (uint32_t)(e->tpr * e->vpt));
 }
 
 // A tile-staged entry runs with a plan that fits (fitting_plan); one on real

@@ -25,6 +25,7 @@
 #include "kpm_multi_real.cuh"
 #include "kpm_multi_tiled.cuh"
 #include "kpm_prefix.cuh"
+#include "kpm_steps.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -248,6 +249,24 @@ bool class_plans(const std::vector<Model *> &models, uint32_t W, const MultiEntr
   return false;
 }
 
+// Whether the register-staged step of a class is the better one: as
+// register_wins of recursion.cu for one model, summed over the class's.  The
+// server's register-staged steps are not dependent launches: they are as fast
+// where the estimates differ by 1.8 (one model of 180k square sites numbered at
+// random, 4 lanes: 30 ms a request tile-staged, 18 register-staged, estimates 50
+// and 17 us a step; 45k sites: 13 and 16 ms, 22 and 13 us).
+bool class_register_wins(const std::vector<Model *> &models, const std::vector<const TilePlan *> &tp,
+                         const MultiEntry *e, bool real) {
+  const int cls = real ? kClassMixedRealDots : kClassMixedDots;
+  const int warps = (e->minb - kMultiTiledVariant) % 1000 / 10;
+  double tiled = 0, registers = 0;
+  for (size_t i = 0; i < models.size(); i++) {
+    tiled += tiled_us(cls, e->tpr, e->vpt, warps, multi_tiled_bps(e->minb), *tp[i], models[i]->mat->device);
+    registers += register_us(models[i]->mat, cls, (uint32_t)(e->tpr * e->vpt));
+  }
+  return tiled > 1.8 * registers;
+}
+
 // Register-staged shape per width and class (few threads per row, several
 // values each): where rows are too narrow for bulk copies, or a model has no
 // plan or no ring that fits.
@@ -372,10 +391,14 @@ struct tbtkkpm_server {
   cudaGraphExec_t tick_exec = nullptr;
   DevBuf d_step;
 
+  std::set<uint32_t> defaults;  // keys of `config` that no one chose
   const std::array<int, 3> &config_for(uint32_t W, bool real) {
     const uint32_t key = W | (real ? 1u << 16 : 0u);
     auto it = config.find(key);
-    if (it == config.end()) it = config.emplace(key, default_config(W, real)).first;
+    if (it == config.end()) {
+      it = config.emplace(key, default_config(W, real)).first;
+      defaults.insert(key);
+    }
     return it->second;
   }
 };
@@ -714,7 +737,8 @@ MultiModel describe(const tbtkkpm_server *s, const Model *m) {
 // Builds the launch plans, one per (lane width, real or complex lanes), of
 // all models with busy lanes (under s->mu).  A class whose configured entry
 // is tile-staged falls back to the default register-staged entry of its
-// width when some model has no plan for it or two ring stages do not fit.
+// width when some model has no plan for it or two ring stages do not fit, and
+// from a default also where that is faster (class_register_wins).
 int plan_tick(tbtkkpm_server *s, std::vector<ClassPlan> &plans) {
   std::map<uint32_t, size_t> index;
   std::vector<std::vector<Model *>> members;
@@ -745,8 +769,10 @@ int plan_tick(tbtkkpm_server *s, std::vector<ClassPlan> &plans) {
     std::vector<const TilePlan *> tp(members[c].size(), nullptr);
     if (is_multi_tiled(cp.entry->minb)) {
       int rc;
-      const bool fits = class_plans(members[c], cp.W, cp.entry, cp.real, tp, cp.ly, &rc);
+      bool fits = class_plans(members[c], cp.W, cp.entry, cp.real, tp, cp.ly, &rc);
       if (rc) return rc;
+      if (s->defaults.count(cp.W | (cp.real ? 1u << 16 : 0u)))
+        fits = fits && !class_register_wins(members[c], tp, cp.entry, cp.real);
       if (!fits) {
         const auto d = register_config(cp.W, cp.real);
         cp.entry = find_multi(d[0], d[1], d[2], cp.real);
@@ -1762,6 +1788,8 @@ extern "C" int tbtkkpm_server_set_config(tbtkkpm_server *s, uint32_t width, int 
   // the lane class(es) this shape is compiled for
   if (cplx) s->config[width] = {tpr, vpt, minb};
   if (real) s->config[width | 1u << 16] = {tpr, vpt, minb};
+  if (cplx) s->defaults.erase(width);
+  if (real) s->defaults.erase(width | 1u << 16);
   return TBTKKPM_OK;
 }
 
@@ -1989,6 +2017,7 @@ int tune_class(tbtkkpm_server *s, Model *probe, uint32_t width, uint32_t probe_s
   if (rc) return rc;
   if (!best) return fail(TBTKKPM_ERR_UNSUPPORTED, "server_autotune: no kernel for width %u", W);
   s->config[W | (real ? 1u << 16 : 0u)] = {best->tpr, best->vpt, best->minb};
+  s->defaults.erase(W | (real ? 1u << 16 : 0u));
   s->tuned.insert(W | (real ? 1u << 16 : 0u));
   // a tile-staged pick: the plans of every model of the class now, not in
   // the first tick that needs them
